@@ -48,9 +48,7 @@ void free_handle(egt_handle* h) {
     cudaSetDevice(h->cfg.device);
     auto F = [h](void* p) { dev_free(h, p); };
     F(h->p4); F(h->p4b); F(h->x); F(h->y); F(h->z); F(h->cell0); F(h->perm); F(h->d_norm);
-    for (int L = 0; L < kMaxLevels; L++) {
-        F(h->lv[L].order); F(h->lv[L].cell_start); F(h->lv[L].cell_x); F(h->lv[L].row_range);
-    }
+    F(h->grid_mem);
     F(h->lists); F(h->kth); F(h->qlevel); F(h->pclass); F(h->csr_off); F(h->csr_col); F(h->tris); F(h->nrm);
     F(h->d_counters); F(h->scratch.ptr);
     if (h->taubin_exec) cudaGraphExecDestroy(h->taubin_exec);
@@ -171,8 +169,8 @@ egt_status create_common(const float* xyz, bool xyz_on_device, int64_t n, const 
     }
     egt_status s = build_grid(h, dxyz, h->is_mesh ? 1 : kMaxLevels);
     if (staged) cudaFreeAsync(staged, h->stream);
+    if (s == EGT_OK) s = fetch_norm(h);  // waits for the build
     if (s != EGT_OK) return fail(s);
-    CREATE_TRY(cudaStreamSynchronize(h->stream));
 #undef CREATE_TRY
     h->tm.grid_ms = elapsed_ms(h->ev[0], h->ev[1]);
     *out = h;
@@ -223,7 +221,10 @@ egt_status egt_update_points_device(egt_handle* h, const float* xyz_dev, void* s
     bind_stream(h, stream);
     h->have_csr = false;
     if (h->nrm) { dev_free(h, h->nrm); h->nrm = nullptr; }
-    return build_grid(h, xyz_dev, kMaxLevels);
+    EGT_TRY(build_grid(h, xyz_dev, kMaxLevels));
+    // the caller may reuse xyz_dev on any stream: it has been read
+    EGT_CUDA_TRY(cudaEventSynchronize(h->ev[kEvRead]));
+    return EGT_OK;
 }
 
 int64_t egt_kernel_launches(void) { return g_launches; }
@@ -492,6 +493,10 @@ egt_status egt_free_device(void* p) {
 egt_status egt_get_views(egt_handle* h, egt_views* v) {
     EGT_TRY(check_handle(h));
     if (!v) { set_error("egt_get_views: null output"); return EGT_ERR_ARG; }
+    if (!h->norm_valid && h->d_norm) {
+        EGT_CUDA_TRY(cudaSetDevice(h->cfg.device));
+        EGT_TRY(fetch_norm(h));
+    }
     v->x = h->x;
     v->y = h->y;
     v->z = h->z;

@@ -40,6 +40,35 @@ void count_launch();
     } while (0)
 
 // ---------------------------------------------------------------------------
+// Programmatic dependent launch (griddepcontrol): wait() blocks until the
+// preceding grid in the stream has completed and its writes are visible (it
+// returns at once when the kernel was not launched as a dependent);
+// launch_dependents() lets the next grid start its prologue on free SMs.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
+
+// Launches `kernel` as a programmatic dependent of the work before it in the
+// stream.  The kernel calls grid_dependency_wait() before it touches memory
+// that earlier work writes or reads.
+template <typename... P, typename... A>
+inline egt_status launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                   A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    EGT_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    EGT_LAUNCH_CHECK();
+    return EGT_OK;
+}
+
+// ---------------------------------------------------------------------------
 // Device rounding shapes.  The reference is built with nvcc's default
 // --fmad=true; these helpers spell out the fused multiply-adds that compiler
 // forms for each expression (identified black-box, see oracle/fp_shapes.h),
@@ -104,7 +133,7 @@ constexpr int kCtrFlag = 27;      // generic loop flag
 constexpr int kCtrNormFallback = 28;  // normals re-solved in FP64
 constexpr int kCtrMsf = 29;       // spanning-forest edges
 constexpr int kCtrComps = 30;     // orientation components
-constexpr int kCtrMaxPop = 32;    // [32..39] largest cell population per level
+constexpr int kCtrMaxPop = 32;    // [32..39] largest cell population per level (grid build)
 constexpr int kCtrBoxTried = 40;  // learned kNN: queries that ran a box search
 constexpr int kCtrCertified = 41; // learned kNN: certified box results
 constexpr int kCtrExactRerun = 42;  // kNN queries re-searched with the exact insertion rule (ties)
@@ -131,6 +160,8 @@ struct LevelDev {
     int2* row_range = nullptr; // [B*B] [first, last) cell of each (y,z) row
 };
 
+constexpr int kEvRead = 16;  // egt_handle::ev
+
 struct Scratch {
     void* ptr = nullptr;
     size_t bytes = 0;
@@ -153,8 +184,11 @@ struct egt_handle {
     uint32_t* cell0 = nullptr;   // [n] packed level-0 cell coords x | y<<10 | z<<20
     int* perm = nullptr;         // [n] sorted -> original
     egt::NormParams* d_norm = nullptr;
-    egt::NormParams norm{};      // host copy
-    egt::LevelDev lv[egt::kMaxLevels];
+    egt::NormParams norm{};      // host copy (fetch_norm)
+    bool norm_valid = false;
+    egt::LevelDev lv[egt::kMaxLevels];  // slices of grid_mem
+    void* grid_mem = nullptr;    // row ranges of all levels, then their cells and orders
+    size_t row_bytes = 0;        // bytes of the row ranges
     int levels_built = 0;
     // neighbourhoods
     int* lists = nullptr;        // [n*k] sorted-space lists
@@ -162,7 +196,6 @@ struct egt_handle {
     uint8_t* qlevel = nullptr;   // [n] level at which each query stopped
     // learned search proposal
     uint8_t* pclass = nullptr;   // [n] proposed class per query
-    bool maxpop_valid = false;   // counters[kCtrMaxPop..] match the current grid
     const egt_proposal* proposal = nullptr;  // attached for knn_mode == EGT_KNN_LEARNED
     bool last_knn_learned = false;
     void* tile_mem = nullptr;    // cell-tile kNN: query levels, unit bits, units, leftover queries
@@ -207,7 +240,7 @@ struct egt_handle {
     const uint16_t* cloud_of = nullptr;
     int cloud_bits = 0;
     // timing
-    cudaEvent_t ev[16] = {};
+    cudaEvent_t ev[17] = {};     // stage timing pairs; kEvRead: the grid build has read its input
     egt_timings tm{};
     egt::Scratch scratch;
 };
@@ -225,6 +258,7 @@ inline void dev_free(egt_handle* h, void* p) {
 }
 egt_status scratch_reserve(egt_handle* h, size_t bytes, void** out);
 egt_status build_grid(egt_handle* h, const float* xyz_dev_aos, int levels);
+egt_status fetch_norm(egt_handle* h);
 egt_status set_threshold(egt_handle* h, float thres);
 egt_status run_knn(egt_handle* h, int k);
 egt_status run_knn_host(egt_handle* h, int k, int* host);

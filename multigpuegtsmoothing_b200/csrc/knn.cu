@@ -720,20 +720,6 @@ egt_status launch_learned(const KnnArgs& a, const uint8_t* cls, cudaStream_t st)
     return EGT_OK;
 }
 
-// Largest cell population of each level (condition (4) above).
-__global__ void k_maxpop(LevelDev lv0, LevelDev lv1, LevelDev lv2, LevelDev lv3, LevelDev lv4, LevelDev lv5,
-                         LevelDev lv6, LevelDev lv7, int n, unsigned long long* __restrict__ counters) {
-    const LevelDev* lvs[kMaxLevels] = {&lv0, &lv1, &lv2, &lv3, &lv4, &lv5, &lv6, &lv7};
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-#pragma unroll
-    for (int L = 0; L < kMaxLevels; L++) {
-        const int nc = (int)counters[kCtrNcells + L];
-        int v = (i < nc && i < n) ? lvs[L]->cell_start[i + 1] - lvs[L]->cell_start[i] : 0;
-        v = __reduce_max_sync(0xffffffffu, v);
-        if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(&counters[kCtrMaxPop + L], (unsigned long long)v);
-    }
-}
-
 template <int S, bool kFast>
 egt_status launch(const KnnArgs& a, cudaStream_t st) {
     unsigned G = 0;
@@ -744,18 +730,6 @@ egt_status launch(const KnnArgs& a, cudaStream_t st) {
 }
 
 }  // namespace
-
-egt_status level_maxpop(egt_handle* h) {
-    if (h->maxpop_valid) return EGT_OK;
-    cudaStream_t st = h->stream;
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrMaxPop, 0, kMaxLevels * sizeof(unsigned long long), st));
-    const unsigned T = 256, G = (unsigned)((h->n + T - 1) / T);
-    k_maxpop<<<G, T, 0, st>>>(h->lv[0], h->lv[1], h->lv[2], h->lv[3], h->lv[4], h->lv[5], h->lv[6], h->lv[7],
-                              (int)h->n, h->d_counters);
-    EGT_LAUNCH_CHECK();
-    h->maxpop_valid = true;
-    return EGT_OK;
-}
 
 // Lists and per-query buffers for k, and the search arguments of handle h.
 static egt_status knn_prepare(egt_handle* h, int k, KnnArgs* a) {
@@ -856,7 +830,6 @@ static egt_status tile_search(egt_handle* h, const KnnArgs& a, cudaStream_t st) 
     t.desc = nullptr;
     t.cloud_of = nullptr;
     t.npts = a.n;
-    EGT_TRY(level_maxpop(h));  // condition (4)
     EGT_TRY(tile_launch<false>(a, t, a.k, st));
     KnnArgs ar = a;
     ar.qmap = t.ring2;
@@ -880,7 +853,6 @@ egt_status run_knn(egt_handle* h, int k) {
         return EGT_OK;
     }
     const bool select = h->cfg.knn_mode == EGT_KNN_SELECT;
-    if (select) EGT_TRY(level_maxpop(h));  // the selection's oversized-cell check
     EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrInvalid, 0, 2 * sizeof(unsigned long long), st));
     EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrExactRerun, 0, 3 * sizeof(unsigned long long), st));
     EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrSelFallback, 0, sizeof(unsigned long long), st));
@@ -977,7 +949,6 @@ egt_status run_knn_host(egt_handle* h, int k, int* host) {
     // per chunk: its work counter and its count of queries the ring search ran
     EGT_CUDA_TRY(cudaMallocAsync((void**)&work, sizeof(unsigned long long) * 2 * chunks, st));
     EGT_CUDA_TRY(cudaMemsetAsync(work, 0, sizeof(unsigned long long) * 2 * chunks, st));
-    if (h->cfg.knn_mode == EGT_KNN_SELECT) EGT_TRY(level_maxpop(h));
     const unsigned T = 256;
     k_chunk_keys<<<(unsigned)((n + T - 1) / T), T, 0, st>>>(h->perm, n, cb, key, idx);
     EGT_LAUNCH_CHECK();
@@ -1148,7 +1119,6 @@ egt_status run_knn_learned(egt_handle* h, int k, const egt_proposal* p) {
     if (!h->qlevel) EGT_CUDA_TRY(dev_alloc(h, &h->qlevel, n));
     h->have_csr = false;
     EGT_CUDA_TRY(cudaEventRecord(h->ev[2], st));
-    EGT_TRY(level_maxpop(h));
     EGT_TRY(proposal_classes(h, p));
     EGT_CUDA_TRY(cudaEventRecord(h->ev[15], st));
     EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrInvalid, 0, 2 * sizeof(unsigned long long), st));

@@ -162,6 +162,5 @@ __device__ __forceinline__ void proposal_features(const LevelDev* lv, const Norm
 // Proposal-network parameters live on the device as binary16 (the weights the
 // kernels compute with); FP32 master copies are kept for training.
 egt_status proposal_classes(egt_handle* h, const egt_proposal* p);  // fills h->pclass
-egt_status level_maxpop(egt_handle* h);                               // fills h->maxpop
 
 }  // namespace egt

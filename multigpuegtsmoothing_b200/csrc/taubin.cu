@@ -97,13 +97,6 @@ __global__ void __launch_bounds__(256) k_taubin(const float4* __restrict__ pin, 
     pout[i] = row_update(pin, col, 0, __ldg(off + i), __ldg(off + i + 1), i, scale);
 }
 
-// Programmatic dependent launch (griddepcontrol): wait() blocks until the
-// preceding grid in the stream has completed and its writes are visible (it
-// returns at once when the kernel was not launched as a dependent);
-// launch_dependents() lets the next grid start its prologue on free SMs.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
-
 constexpr int kUCap = 1024;      // distinct neighbours staged per tile (16 KB; 99.8% of tiles fit)
 constexpr int kUPer = kUCap / kTile;  // staged positions per thread
 constexpr int kSlices = kTile / 32;   // one 32-row slice per warp
