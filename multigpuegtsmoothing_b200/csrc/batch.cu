@@ -253,6 +253,7 @@ struct DescArgs {
     float* kth;
     uint8_t* qlevel;
     unsigned long long* ctr;
+    bool jump;
 };
 
 __global__ void k_make_desc(DescArgs d, KnnArgs* __restrict__ out) {
@@ -280,8 +281,23 @@ __global__ void k_make_desc(DescArgs d, KnnArgs* __restrict__ out) {
     a.kth_out = d.kth + o;
     a.qlevel = d.qlevel + o;
     a.counters = d.ctr + (size_t)c * kCtrWords;
+    a.maxpop = a.counters + kCtrMaxPop;
     a.gbase = o;
+    a.jump = d.jump;
     out[c] = a;
+}
+
+// Largest cell population of each cloud and level (the searches' oversized-cell
+// check): blockIdx.x a slice of the cells, (y, z) the level and the cloud.
+constexpr int kPopSlices = 16;
+__global__ void __launch_bounds__(256) k_maxpop_batch(const KnnArgs* __restrict__ desc) {
+    const KnnArgs& a = desc[blockIdx.z];
+    const LevelDev& LV = a.lv[blockIdx.y];
+    int v = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < LV.ncells; i += kPopSlices * blockDim.x)
+        v = max(v, LV.cell_start[i + 1] - LV.cell_start[i]);
+    v = __reduce_max_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(&a.counters[kCtrMaxPop + blockIdx.y], (unsigned long long)v);
 }
 
 __global__ void k_set_chunk(KnnArgs* __restrict__ desc, int count, int chunk) {
@@ -482,18 +498,6 @@ egt_status launch_compact_batch(egt_batch* b, cudaStream_t st) {
     return EGT_OK;
 }
 
-// Blocks of one resident wave of k_knn_batch<S>.
-// Largest cell population of each cloud and level (the cell-tile search's
-// oversized-cell check): block (cloud, level).
-__global__ void __launch_bounds__(256) k_maxpop_batch(const KnnArgs* __restrict__ desc) {
-    const KnnArgs& a = desc[blockIdx.x];
-    const LevelDev& LV = a.lv[blockIdx.y];
-    int v = 0;
-    for (int i = threadIdx.x; i < LV.ncells; i += blockDim.x) v = max(v, LV.cell_start[i + 1] - LV.cell_start[i]);
-    v = __reduce_max_sync(0xffffffffu, v);
-    if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(&a.counters[kCtrMaxPop + blockIdx.y], (unsigned long long)v);
-}
-
 // The ring search of the queries in `list` (indices over all clouds' points),
 // one query per warp.
 template <int S>
@@ -526,6 +530,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_knn_list_batch(const KnnArgs* _
     }
 }
 
+// Blocks of one resident wave of k_knn_batch<S>.
 template <int S>
 egt_status knn_wave(int device, unsigned* out) {
     static std::mutex mu;
@@ -603,10 +608,6 @@ egt_status knn_batch_tile(egt_batch* b, cudaStream_t st) {
     t.desc = b->d_desc;
     t.cloud_of = b->d_cloud;
     t.npts = (int)b->N;
-    EGT_CUDA_TRY(cudaMemset2DAsync(b->d_ctr + kCtrMaxPop, sizeof(unsigned long long) * kCtrWords, 0,
-                                   kMaxLevels * sizeof(unsigned long long), b->count, st));
-    k_maxpop_batch<<<dim3(b->count, kMaxLevels), 256, 0, st>>>(b->d_desc);
-    EGT_LAUNCH_CHECK();
     int kt = 0;  // the largest k the tile search takes
     for (int c = 0; c < b->count; c++)
         if (b->k[c] >= kTileMinK && b->k[c] <= kTileMaxK) kt = std::max(kt, b->k[c]);
@@ -1026,7 +1027,10 @@ egt_status egt_batch_create(const float* xyz_host, const int64_t* offsets, const
     da.kth = h->kth;
     da.qlevel = h->qlevel;
     da.ctr = b->d_ctr;
+    da.jump = cfg.knn_mode != EGT_KNN_PLAIN;
     k_make_desc<<<blocks(count), kB, 0, st>>>(da, b->d_desc);
+    BSTAT([&] { EGT_LAUNCH_CHECK(); return EGT_OK; }());
+    k_maxpop_batch<<<dim3(kPopSlices, kMaxLevels, (unsigned)count), 256, 0, st>>>(b->d_desc);
     BSTAT([&] { EGT_LAUNCH_CHECK(); return EGT_OK; }());
     BTRY(cudaEventRecord(h->ev[1], st));
     for (void* p : {(void*)dxyz, (void*)acc, (void*)tmp4, (void*)kA, (void*)kB2, (void*)iA, (void*)iB, (void*)flag,

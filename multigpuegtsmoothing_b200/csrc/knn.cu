@@ -56,8 +56,9 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_knn_plain(KnnArgs a
     const NormParams np = *a.np;
     unsigned evals = 0;  // candidate distances this lane evaluated
     const int n = launch_size(a);
-    for (int q0 = claim(a, lane, n); q0 < n; q0 = claim(a, lane, n)) {
-        const int q1 = min(q0 + a.chunk, n);
+    const int chunk = claim_chunk(a, n);
+    for (int q0 = claim(a, lane, n, chunk); q0 < n; q0 = claim(a, lane, n, chunk)) {
+        const int q1 = min(q0 + chunk, n);
         for (int jq = q0; jq < q1; jq++) {
             const int q = a.qmap ? a.qmap[jq] : jq;
             const float4 pq = a.p4[q];
@@ -92,8 +93,9 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_knn_select(KnnArgs 
     const int n = launch_size(a);
     unsigned evals = 0, ring = 0, reruns = 0;
     int gstart = 0, maxlevel = 0;
-    for (int q0 = claim(a, lane, n); q0 < n; q0 = claim(a, lane, n)) {
-        const int q1 = min(q0 + a.chunk, n);
+    const int chunk = a.chunk;  // consecutive queries share their level
+    for (int q0 = claim(a, lane, n, chunk); q0 < n; q0 = claim(a, lane, n, chunk)) {
+        const int q1 = min(q0 + chunk, n);
         for (int jq = q0; jq < q1; jq++) {
             const int q = a.qmap ? a.qmap[jq] : jq;
             const float4 pq = a.p4[q];
@@ -508,8 +510,9 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_knn_learned(KnnArgs
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const NormParams np = *a.np;
     const int n = launch_size(a);
-    for (int q0 = claim(a, lane, n); q0 < n; q0 = claim(a, lane, n)) {
-        const int q1 = min(q0 + a.chunk, n);
+    const int chunk = claim_chunk(a, n);
+    for (int q0 = claim(a, lane, n, chunk); q0 < n; q0 = claim(a, lane, n, chunk)) {
+        const int q1 = min(q0 + chunk, n);
         for (int jq = q0; jq < q1; jq++) {
             const int q = a.qmap ? a.qmap[jq] : jq;
             const float4 pq = a.p4[q];
@@ -580,21 +583,39 @@ __device__ int search_query(const KnnArgs& a, const NormParams& np, float4 pq, c
     L.init(kExact ? k : k + 1);
     invalid = false;
     int ci[3], cp[3];
+    auto cells = [&](int lvl) {
 #pragma unroll
-    for (int d = 0; d < 3; d++) ci[d] = (int)__fmul_rn(u[d], 1024.0f);
-    int2 own = lane == 0 ? find_cell(a.lv[0], ci[0], ci[1], ci[2]) : make_int2(-1, -1);
-    stream_cells<kExact, S>(L, invalid, 1, own.x, own.y, nullptr, a.p4, -1, pq, thres_lt, a.max_pts, lane, -1, 0, 0,
-                            0, s_pref, s_start, s_md, s_mp);
-    bool cont = decide_query(np, 0, 0, L.counter, k, kExact ? L.kth : L.fetch_dist(k - 1), invalid, pq, ci);
-    int reached = 0;
-    for (int lvl = 0; cont; lvl++) {
+        for (int d = 0; d < 3; d++) ci[d] = (int)__fmul_rn(u[d], (float)(1024 >> lvl));
+    };
+    // Inside the reference's cube the cells of a query nest (the products are
+    // exact), so its search may start at the first level that can fill the
+    // list (first_full_level; no point is excluded here).
+    int2 first = make_int2(-1, -1);
+    int l1 = -1;
+    bool inside = !kExact && np.thres > 4.0f;
+#pragma unroll
+    for (int d = 0; d < 3; d++) inside = inside && u[d] >= 0.0f && u[d] < 1.0f;
+    if (inside) {
+        l1 = first_full_level(a, k, [&](int l) {
+            const float B = (float)(1024 >> l);
+            return make_int3((int)__fmul_rn(u[0], B), (int)__fmul_rn(u[1], B), (int)__fmul_rn(u[2], B));
+        }, lane, first);
+        if (l1 >= 0 && a.maxpop[l1] >= (unsigned long long)a.max_pts) l1 = -1;
+    }
+    cells(max(l1, 0));
+    if (l1 < 0) first = lane == 0 ? find_cell(a.lv[0], ci[0], ci[1], ci[2]) : make_int2(-1, -1);
+    stream_cells<kExact, S>(L, invalid, l1 < 0 ? 1 : 32, first.x, first.y, l1 < 0 ? nullptr : a.lv[l1].order, a.p4, -1,
+                            pq, thres_lt, l1 < 0 ? a.max_pts : INT_MAX, lane, -1, 0, 0, 0, s_pref, s_start, s_md,
+                            s_mp);
+    bool cont = decide_query(np, max(l1, 0), l1 < 0 ? 0 : 1, L.counter, k, kExact ? L.kth : L.fetch_dist(k - 1),
+                             invalid, pq, ci);
+    int reached = max(l1, 0);
+    for (int lvl = l1 + 1; cont && lvl < kMaxLevels; lvl++) {
         reached = lvl;
         const LevelDev& LV = a.lv[lvl];
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-            cp[d] = (int)__fmul_rn(u[d], (float)(1024 >> max(lvl - 1, 0)));  // the block visited so far
-            ci[d] = (int)__fmul_rn(u[d], (float)(1024 >> lvl));
-        }
+        for (int d = 0; d < 3; d++) cp[d] = (int)__fmul_rn(u[d], (float)(1024 >> max(lvl - 1, 0)));  // visited so far
+        cells(lvl);
         int2 cell = make_int2(-1, -1);
         bool culled = false;
         if (lane < 26) {
@@ -605,7 +626,6 @@ __device__ int search_query(const KnnArgs& a, const NormParams& np, float4 pq, c
         stream_cells<kExact, S>(L, invalid, 26, cell.x, cell.y, LV.order, a.p4, -1, pq, thres_lt, a.max_pts, lane,
                                 lvl - 1, cp[0], cp[1], cp[2], s_pref, s_start, s_md, s_mp, culled);
         cont = decide_query(np, lvl, 1, L.counter, k, kExact ? L.kth : L.fetch_dist(k - 1), invalid, pq, ci);
-        if (lvl == kMaxLevels - 1) break;
     }
     if (cont) { invalid = true; reached = kMaxLevels; }
     return reached;
@@ -627,8 +647,9 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_knn_query(KnnArgs a
     const float thres_lt = nextafterf(np.thres, 0.0f);  // d <= thres_lt  <=>  d < thres
     const float ab = __fsub_rn(np.b, np.a);
     const int n = launch_size(a);
-    for (int q0 = claim(a, lane, n); q0 < n; q0 = claim(a, lane, n)) {
-        const int q1 = min(q0 + a.chunk, n);
+    const int chunk = claim_chunk(a, n);
+    for (int q0 = claim(a, lane, n, chunk); q0 < n; q0 = claim(a, lane, n, chunk)) {
+        const int q1 = min(q0 + chunk, n);
         for (int jq = q0; jq < q1; jq++) {
             const int row = a.qmap[jq];
             const float4 pq = qpos[row];
@@ -698,7 +719,7 @@ egt_status wave_blocks(K kernel, int64_t n, unsigned* out, size_t dyn_smem = 0) 
         std::lock_guard<std::mutex> lock(mu);
         cache[key] = blocks;
     }
-    const int64_t need = (n + kWarps * kChunk - 1) / (kWarps * kChunk);  // enough for the default chunk
+    const int64_t need = (n + kWarps - 1) / kWarps;  // a query per warp
     *out = (unsigned)std::max<int64_t>(1, std::min<int64_t>(blocks, need));
     return EGT_OK;
 }
@@ -756,7 +777,9 @@ static egt_status knn_prepare(egt_handle* h, int k, KnnArgs* a) {
     a->kth_out = h->kth;
     a->qlevel = h->qlevel;
     a->counters = h->d_counters;
+    a->maxpop = h->d_counters + kCtrMaxPop;
     a->qmap = nullptr;
+    a->jump = h->cfg.knn_mode != EGT_KNN_PLAIN;
     return EGT_OK;
 }
 
@@ -1083,6 +1106,7 @@ egt_status run_knn_query(egt_handle* h, const float* q_host, int64_t nq, int k, 
     a.kth_out = nullptr;
     a.qlevel = nullptr;
     a.counters = ctr;
+    a.maxpop = h->d_counters + kCtrMaxPop;
     a.qmap = qmap;
     egt_status s;
     if (k + 1 <= 32) s = launch_query<1>(a, qpos, h->perm, out, st);
@@ -1136,6 +1160,7 @@ egt_status run_knn_learned(egt_handle* h, int k, const egt_proposal* p) {
     a.kth_out = h->kth;
     a.qlevel = h->qlevel;
     a.counters = h->d_counters;
+    a.maxpop = h->d_counters + kCtrMaxPop;
     if (k + 1 <= 32) EGT_TRY(launch_learned<1>(a, h->pclass, st));
     else if (k + 1 <= 64) EGT_TRY(launch_learned<2>(a, h->pclass, st));
     else if (k + 1 <= 96) EGT_TRY(launch_learned<3>(a, h->pclass, st));

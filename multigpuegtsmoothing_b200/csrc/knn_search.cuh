@@ -5,6 +5,7 @@
 #include <climits>
 #include "egt_internal.cuh"
 #include "knn_common.cuh"
+#include "proposal.cuh"
 
 namespace egt {
 namespace {
@@ -19,6 +20,11 @@ struct KnnArgs {
     float* __restrict__ kth_out;
     uint8_t* __restrict__ qlevel;
     unsigned long long* __restrict__ counters;
+    const unsigned long long* __restrict__ maxpop = nullptr;  // [kMaxLevels] largest cell population of each level
+    // The search may start at the first level that can fill the list
+    // (first_full_level).  Off for EGT_KNN_PLAIN, which takes the reference's
+    // steps one by one: the other modes' speed is judged against it.
+    bool jump = true;
     const int* __restrict__ qmap = nullptr;  // query j of a launch is qmap[j] (nullptr: j)
     unsigned long long* __restrict__ work = nullptr;  // work counter (nullptr: counters[kCtrWork])
     const unsigned long long* __restrict__ n_dev = nullptr;  // launch size on the device (nullptr: n)
@@ -254,12 +260,50 @@ __device__ __forceinline__ void stream_cells(WarpList<S>& L, bool& invalid, int 
     if (bigmask) invalid = true;
 }
 
+// The level at which the search of a query can first fill its list: the first
+// whose 3x3x3 block around the query's cell (ci(L)) holds at least `need`
+// points, and that block's nine row ranges, one per lane (nearest rows first).
+// Every earlier step leaves the list short, and a short list always continues
+// when the threshold admits every distance (thres > 4 for points of the unit
+// cube: some face of a block lies inside the grid at every level, nearer than
+// sqrt(thres)).  So the search may start with this block, whatever order its
+// points come in, as long as the order of equal distances does not matter and
+// no cell up to this level is oversized.  Blocks are counted three levels at a
+// time, a row per lane: the levels one by one cost a chain of dependent
+// lookups each (for 2,000 points, k = 10, the whole search took 71 us).
+// Returns -1 when no level has such a block (or the own cell may fill the list
+// on its own: level 0).
+template <typename CI>
+__device__ __forceinline__ int first_full_level(const KnnArgs& a, int need, CI&& ci, int lane, int2& range) {
+#pragma unroll 1
+    for (int l0 = 0; l0 < kMaxLevels; l0 += 3) {
+        const int g = lane / 9, l = l0 + g;
+        int2 rg = make_int2(0, 0);
+        if (lane < 27 && l < kMaxLevels) {
+            const int3 c = ci(l);
+            const int r = lane - 9 * g;
+            rg = row_points(a.lv[l], c.x - 1, c.x + 1, c.y + kRowOrder[r][0], c.z + kRowOrder[r][1]);
+        }
+        const int sz = rg.y - rg.x;
+        int sel = -1;
+#pragma unroll
+        for (int i = 2; i >= 0; i--)
+            if (__reduce_add_sync(0xffffffffu, g == i ? sz : 0) >= need) sel = i;
+        if (sel < 0) continue;
+        if (l0 + sel == 0) return -1;
+        range = g == sel ? rg : make_int2(0, 0);
+        return l0 + sel;
+    }
+    return -1;
+}
+
 // The whole reference search for query q.  Returns the level reached
 // (kMaxLevels when the query ran out of levels).  kExact keeps the k-slot
 // list of the reference's insertion rule; otherwise the list keeps k+1 slots
 // (one more than the output) so that has_ties can check the k-th/(k+1)-th
-// boundary.  Either way the decisions see the k-th smallest distance offered
-// so far, which does not depend on the insertion rule.
+// boundary, and the steps that cannot fill the list are taken as one
+// (first_full_level).  Either way the decisions see the k-th smallest distance
+// offered so far, which does not depend on the insertion rule.
 template <bool kExact, int S>
 __device__ int search(const KnnArgs& a, const NormParams& np, int q, float4 pq, WarpList<S>& L,
                       bool& invalid, int lane, int* s_pref, int* s_start, float* s_md, int* s_mp) {
@@ -268,13 +312,21 @@ __device__ int search(const KnnArgs& a, const NormParams& np, int q, float4 pq, 
     const int k = a.k;
     L.init(kExact ? k : k + 1);
     invalid = false;
+    int2 first = make_int2(-1, -1);
+    int l1 = -1;  // the level to start at (-1: the query's own level-0 cell)
+    if (!kExact && a.jump && np.thres > 4.0f) {
+        l1 = first_full_level(a, k + 1, [&](int l) { return make_int3(cx0 >> l, cy0 >> l, cz0 >> l); }, lane, first);
+        if (l1 >= 0 && a.maxpop[l1] >= (unsigned long long)a.max_pts) l1 = -1;  // populations grow with the level
+    }
     // offset 0 at level 0: the query's own cell (always occupied)
-    int2 own = lane == 0 ? find_cell(a.lv[0], cx0, cy0, cz0) : make_int2(-1, -1);
-    stream_cells<kExact, S>(L, invalid, 1, own.x, own.y, nullptr, a.p4, q, pq, np.thres, a.max_pts, lane, -1, 0, 0, 0,
-                            s_pref, s_start, s_md, s_mp);
-    bool cont = decide(np, 0, 0, L.counter, k, kExact ? L.kth : L.fetch_dist(k - 1), invalid, pq, cx0, cy0, cz0);
-    int reached = 0;
-    for (int lvl = 0; cont; lvl++) {
+    if (l1 < 0) first = lane == 0 ? find_cell(a.lv[0], cx0, cy0, cz0) : make_int2(-1, -1);
+    stream_cells<kExact, S>(L, invalid, l1 < 0 ? 1 : 32, first.x, first.y, l1 < 0 ? nullptr : a.lv[l1].order, a.p4, q,
+                            pq, np.thres, l1 < 0 ? a.max_pts : INT_MAX, lane, -1, 0, 0, 0, s_pref, s_start, s_md,
+                            s_mp);
+    bool cont = decide(np, max(l1, 0), l1 < 0 ? 0 : 1, L.counter, k, kExact ? L.kth : L.fetch_dist(k - 1), invalid, pq,
+                       cx0, cy0, cz0);
+    int reached = max(l1, 0);
+    for (int lvl = l1 + 1; cont && lvl < kMaxLevels; lvl++) {
         reached = lvl;
         const LevelDev& LV = a.lv[lvl];
         int2 cell = make_int2(-1, -1);
@@ -289,7 +341,6 @@ __device__ int search(const KnnArgs& a, const NormParams& np, int q, float4 pq, 
         stream_cells<kExact, S>(L, invalid, 26, cell.x, cell.y, LV.order, a.p4, q, pq, np.thres, a.max_pts, lane,
                                 lvl - 1, cx0 >> sL, cy0 >> sL, cz0 >> sL, s_pref, s_start, s_md, s_mp, culled);
         cont = decide(np, lvl, 1, L.counter, k, kExact ? L.kth : L.fetch_dist(k - 1), invalid, pq, cx0, cy0, cz0);
-        if (lvl == kMaxLevels - 1) break;
     }
     // still searching after the B = 8 ring: invalid (GridKNNCuda.cu:2572-2586)
     if (cont) { invalid = true; reached = kMaxLevels; }
@@ -334,10 +385,16 @@ __device__ __forceinline__ void write_query(const KnnArgs& a, int q, const WarpL
 // atomic (KnnArgs::chunk).
 constexpr int kChunk = 4;
 
+// Queries per claim: one while a launch has few for each warp, so that no warp
+// runs several one after the other while others idle.
+__device__ __forceinline__ int claim_chunk(const KnnArgs& a, int n) {
+    return n > 16 * (int)((gridDim.x * blockDim.x) >> 5) ? a.chunk : 1;
+}
+
 // Next chunk of queries for the calling warp (uniform); >= n when done.
-__device__ __forceinline__ int claim(const KnnArgs& a, int lane, int n) {
+__device__ __forceinline__ int claim(const KnnArgs& a, int lane, int n, int chunk) {
     unsigned long long q0 = 0;
-    if (lane == 0) q0 = atomicAdd(a.work ? a.work : &a.counters[kCtrWork], (unsigned long long)a.chunk);
+    if (lane == 0) q0 = atomicAdd(a.work ? a.work : &a.counters[kCtrWork], (unsigned long long)chunk);
     return (int)min(__shfl_sync(0xffffffffu, q0, 0), (unsigned long long)n);
 }
 
