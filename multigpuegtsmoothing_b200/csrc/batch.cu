@@ -625,11 +625,9 @@ egt_status knn_batch(egt_batch* b) {
     cudaStream_t st = b->h->stream;
     EGT_TRY(set_chunk(b, b->chunk > 0 ? b->chunk : kChunk));
     // reset every cloud's kNN counters and the shared work counter
-    EGT_CUDA_TRY(cudaMemsetAsync(b->h->d_counters + kCtrWork, 0, sizeof(unsigned long long), st));
-    EGT_CUDA_TRY(cudaMemset2DAsync(b->d_ctr + kCtrInvalid, sizeof(unsigned long long) * kCtrWords, 0,
-                                   2 * sizeof(unsigned long long), b->count, st));
-    EGT_CUDA_TRY(cudaMemset2DAsync(b->d_ctr + kCtrExactRerun, sizeof(unsigned long long) * kCtrWords, 0,
-                                   sizeof(unsigned long long), b->count, st));
+    EGT_TRY(reset_knn_counters(b->h));
+    EGT_CUDA_TRY(cudaMemset2DAsync(b->d_ctr + kCtrKnn, sizeof(unsigned long long) * kCtrWords, 0,
+                                   kCtrKnnWords * sizeof(unsigned long long), b->count, st));
     EGT_CUDA_TRY(cudaEventRecord(b->h->ev[2], st));
     const int kk = b->kmax;
     bool tile = b->cfg.knn_mode == EGT_KNN_TILE;
@@ -711,11 +709,9 @@ egt_status knn_egt_batch(egt_batch* b, float alpha) {
     cudaStream_t st = b->h->stream;
     const int64_t N = b->N;
     EGT_TRY(set_chunk(b, b->chunk > 0 ? b->chunk : kChunk));
-    EGT_CUDA_TRY(cudaMemsetAsync(b->h->d_counters + kCtrWork, 0, sizeof(unsigned long long), st));
-    EGT_CUDA_TRY(cudaMemset2DAsync(b->d_ctr + kCtrInvalid, sizeof(unsigned long long) * kCtrWords, 0,
-                                   2 * sizeof(unsigned long long), b->count, st));
-    EGT_CUDA_TRY(cudaMemset2DAsync(b->d_ctr + kCtrExactRerun, sizeof(unsigned long long) * kCtrWords, 0,
-                                   sizeof(unsigned long long), b->count, st));
+    EGT_TRY(reset_knn_counters(b->h));
+    EGT_CUDA_TRY(cudaMemset2DAsync(b->d_ctr + kCtrKnn, sizeof(unsigned long long) * kCtrWords, 0,
+                                   kCtrKnnWords * sizeof(unsigned long long), b->count, st));
     int* counts = nullptr;
     EGT_CUDA_TRY(cudaMallocAsync((void**)&counts, sizeof(int) * (N + 1), st));
     EGT_CUDA_TRY(cudaMemsetAsync(counts + N, 0, sizeof(int), st));

@@ -126,28 +126,29 @@ constexpr int kMaxLevels = 8;  // levels 0..7 (B = 1024 .. 8) are searched
 constexpr int kCtrWords = 64;
 constexpr int kCtrNcells = 0;     // [0..7]  occupied cells per level (int in a u64 slot)
 constexpr int kCtrExtents = 16;   // [16..18] six packed u32 min/max words
-constexpr int kCtrInvalid = 24;   // invalid queries of the last kNN
-constexpr int kCtrMaxLevel = 25;  // deepest level reached
-constexpr int kCtrNnz = 26;       // EGT kept neighbours
+constexpr int kCtrEgtTests = 24;    // EGT filter: ellipsoid tests of the last filter run
+constexpr int kCtrSpillTiles = 25;  // Taubin tiles that gather from global memory (too large to stage)
 constexpr int kCtrFlag = 27;      // generic loop flag
 constexpr int kCtrNormFallback = 28;  // normals re-solved in FP64
 constexpr int kCtrMsf = 29;       // spanning-forest edges
 constexpr int kCtrComps = 30;     // orientation components
 constexpr int kCtrMaxPop = 32;    // [32..39] largest cell population per level (grid build)
-constexpr int kCtrBoxTried = 40;  // learned kNN: queries that ran a box search
-constexpr int kCtrCertified = 41; // learned kNN: certified box results
-constexpr int kCtrExactRerun = 42;  // kNN queries re-searched with the exact insertion rule (ties)
-constexpr int kCtrWork = 43;        // work queue of the persistent kNN kernels (reset with 42)
-constexpr int kCtrEvals = 44;       // plain kNN: candidate distances evaluated (reset with 42)
-constexpr int kCtrEgtTests = 45;    // EGT filter: ellipsoid tests of the last filter run
-constexpr int kCtrSpillTiles = 46;  // Taubin tiles that gather from global memory (too large to stage)
-constexpr int kCtrSelFallback = 48; // queries the selection kNN could not certify (the ring search ran them)
-constexpr int kCtrTileUnits = 49;    // cell-tile kNN: units (level, cell) to search
-constexpr int kCtrTileWork = 50;     // cell-tile kNN: next unit to claim
-constexpr int kCtrTileRingWork = 51; // cell-tile kNN: work counter of the ring search over its leftovers
-constexpr int kCtrTileQ = 52;        // cell-tile kNN: queries compacted by unit
-constexpr int kCtrTileRing2 = 55;    // cell-tile kNN: queries it could not certify (the ring search ran them)
-constexpr int kCtrTileRingWork1 = 56; // cell-tile kNN: next unselected query for the ring search in the tile kernel
+// counters of the last kNN, reset together
+constexpr int kCtrKnn = 40, kCtrKnnWords = 14;
+constexpr int kCtrInvalid = 40;     // invalid queries
+constexpr int kCtrMaxLevel = 41;    // deepest level reached
+constexpr int kCtrExactRerun = 42;  // queries re-searched with the exact insertion rule (ties)
+constexpr int kCtrWork = 43;        // work queue of the persistent kernels
+constexpr int kCtrEvals = 44;       // plain kNN: candidate distances evaluated
+constexpr int kCtrSelFallback = 45; // queries the selection kNN could not certify (the ring search ran them)
+constexpr int kCtrTileUnits = 46;    // cell-tile kNN: units (level, cell) to search
+constexpr int kCtrTileWork = 47;     // cell-tile kNN: next unit to claim
+constexpr int kCtrTileRingWork = 48; // cell-tile kNN: work counter of the ring search over its leftovers
+constexpr int kCtrTileQ = 49;        // cell-tile kNN: queries compacted by unit
+constexpr int kCtrTileRing2 = 50;    // cell-tile kNN: queries it could not certify (the ring search ran them)
+constexpr int kCtrTileRingWork1 = 51; // cell-tile kNN: next unselected query for the ring search in the tile kernel
+constexpr int kCtrBoxTried = 52;    // learned kNN: queries that ran a box search
+constexpr int kCtrCertified = 53;   // learned kNN: certified box results
 
 // One level of the cell hierarchy.  Cells are sorted by key
 // x + y*B + z*B^2; a row is the set of occupied cells sharing (y, z).
@@ -259,6 +260,10 @@ inline void dev_free(egt_handle* h, void* p) {
 egt_status scratch_reserve(egt_handle* h, size_t bytes, void** out);
 egt_status build_grid(egt_handle* h, const float* xyz_dev_aos, int levels);
 egt_status fetch_norm(egt_handle* h);
+inline egt_status reset_knn_counters(egt_handle* h) {
+    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrKnn, 0, kCtrKnnWords * sizeof(unsigned long long), h->stream));
+    return EGT_OK;
+}
 egt_status set_threshold(egt_handle* h, float thres);
 egt_status run_knn(egt_handle* h, int k);
 egt_status run_knn_host(egt_handle* h, int k, int* host);

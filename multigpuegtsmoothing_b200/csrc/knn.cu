@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_knn_plain(KnnArgs a
     if (threadIdx.x == 0) s_rerun = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    grid_dependency_wait();
     const NormParams np = *a.np;
     unsigned evals = 0;  // candidate distances this lane evaluated
     const int n = launch_size(a);
@@ -745,9 +746,7 @@ template <int S, bool kFast>
 egt_status launch(const KnnArgs& a, cudaStream_t st) {
     unsigned G = 0;
     EGT_TRY(wave_blocks(k_knn_plain<S, kFast>, a.n, &G));
-    k_knn_plain<S, kFast><<<G, kWarps * 32, 0, st>>>(a);
-    EGT_LAUNCH_CHECK();
-    return EGT_OK;
+    return launch_dependent(k_knn_plain<S, kFast>, dim3(G), dim3(kWarps * 32), 0, st, a);
 }
 
 }  // namespace
@@ -865,23 +864,10 @@ egt_status run_knn(egt_handle* h, int k) {
     cudaStream_t st = h->stream;
     KnnArgs a;
     EGT_TRY(knn_prepare(h, k, &a));
-    if (h->cfg.knn_mode == EGT_KNN_TILE && k >= kTileMinK && k <= kTileMaxK) {
-        EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrInvalid, 0, 2 * sizeof(unsigned long long), st));
-        EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrExactRerun, 0, 3 * sizeof(unsigned long long), st));
-        EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrSelFallback, 0, sizeof(unsigned long long), st));
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrTileRing2, 0, sizeof(unsigned long long), st));
-        EGT_CUDA_TRY(cudaEventRecord(h->ev[2], st));
-        EGT_TRY(tile_search(h, a, st));
-        EGT_CUDA_TRY(cudaEventRecord(h->ev[3], st));
-        return EGT_OK;
-    }
-    const bool select = h->cfg.knn_mode == EGT_KNN_SELECT;
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrInvalid, 0, 2 * sizeof(unsigned long long), st));
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrExactRerun, 0, 3 * sizeof(unsigned long long), st));
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrSelFallback, 0, sizeof(unsigned long long), st));
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrTileRing2, 0, sizeof(unsigned long long), st));
+    EGT_TRY(reset_knn_counters(h));
     EGT_CUDA_TRY(cudaEventRecord(h->ev[2], st));
-    EGT_TRY(knn_search(a, select, st));
+    if (h->cfg.knn_mode == EGT_KNN_TILE && k >= kTileMinK && k <= kTileMaxK) EGT_TRY(tile_search(h, a, st));
+    else EGT_TRY(knn_search(a, h->cfg.knn_mode == EGT_KNN_SELECT, st));
     EGT_CUDA_TRY(cudaEventRecord(h->ev[3], st));
     return EGT_OK;
 }
@@ -980,11 +966,7 @@ egt_status run_knn_host(egt_handle* h, int k, int* host) {
     void* tmp = nullptr;
     EGT_TRY(scratch_reserve(h, t_sort, &tmp));
     EGT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, t_sort, key, key2, idx, qmap, n, 0, bits, st));
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrInvalid, 0, 2 * sizeof(unsigned long long), st));
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrExactRerun, 0, sizeof(unsigned long long), st));
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrEvals, 0, sizeof(unsigned long long), st));
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrSelFallback, 0, sizeof(unsigned long long), st));
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrTileRing2, 0, sizeof(unsigned long long), st));
+    EGT_TRY(reset_knn_counters(h));
     EGT_CUDA_TRY(cudaEventRecord(h->ev[2], st));
     // streams: [0] = h->stream, [1] = a second search stream, [2] = copies
     cudaStream_t ss[3] = {st, nullptr, nullptr};
@@ -1145,9 +1127,7 @@ egt_status run_knn_learned(egt_handle* h, int k, const egt_proposal* p) {
     EGT_CUDA_TRY(cudaEventRecord(h->ev[2], st));
     EGT_TRY(proposal_classes(h, p));
     EGT_CUDA_TRY(cudaEventRecord(h->ev[15], st));
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrInvalid, 0, 2 * sizeof(unsigned long long), st));
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrBoxTried, 0, 2 * sizeof(unsigned long long), st));
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrExactRerun, 0, 3 * sizeof(unsigned long long), st));
+    EGT_TRY(reset_knn_counters(h));
     KnnArgs a;
     a.p4 = h->p4;
     a.np = h->d_norm;

@@ -171,6 +171,8 @@ __device__ __forceinline__ void warp_append64(bool flag, unsigned long long v, u
 // all clouds (their sorted order).
 template <bool kBatch>
 __global__ void __launch_bounds__(256) k_tile_assign(KnnArgs a, TileArgs t) {
+    grid_dependency_wait();
+    grid_dependents_launch();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const bool in = i < t.npts;
@@ -250,6 +252,8 @@ __device__ __forceinline__ int tile_class(int pop) {
 // and the batch count of each class.
 template <bool kBatch>
 __global__ void __launch_bounds__(256) k_tile_count(KnnArgs a, TileArgs t) {
+    grid_dependency_wait();
+    grid_dependents_launch();
     const int lane = threadIdx.x & 31;
     const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nw = (int)((gridDim.x * blockDim.x) >> 5);
@@ -293,6 +297,8 @@ __global__ void __launch_bounds__(256) k_tile_count(KnnArgs a, TileArgs t) {
 // 16 (one warp per unit, grid-stride), the batches ordered by class.
 template <bool kBatch>
 __global__ void __launch_bounds__(256) k_tile_gather(KnnArgs a, TileArgs t) {
+    grid_dependency_wait();
+    grid_dependents_launch();
     const int lane = threadIdx.x & 31;
     const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nw = (int)((gridDim.x * blockDim.x) >> 5);
@@ -520,6 +526,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, 16) k_knn_tile(KnnArgs a, Til
     constexpr int kCap = tile_cap<S>();
     constexpr size_t kWarpBytes = tile_warp_bytes<S>();
     extern __shared__ __align__(16) unsigned char s_tile[];
+    grid_dependency_wait();
+    grid_dependents_launch();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int hl = lane & 15, hf = lane >> 4;
     unsigned char* base = s_tile + (size_t)w * kWarpBytes;
@@ -788,7 +796,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 16) k_knn_tile(KnnArgs a, Til
 
 
 // Working buffers of the cell-tile search for the handle's n points (all
-// clouds' points for a batch), and its counters reset.
+// clouds' points for a batch).  The kNN counters are reset by the caller.
 inline egt_status tile_prepare(egt_handle* h, TileArgs* t) {
     const int64_t n = h->n;
     const int words = (int)((n + 31) / 32);
@@ -810,11 +818,11 @@ inline egt_status tile_prepare(egt_handle* h, TileArgs* t) {
     t->cls_n = tctr;
     t->cls_fill = tctr + kTileClasses;
     m += b_ctr;
-    t->lq = m;
-    m += b_lq;
     t->unit_bits = reinterpret_cast<uint32_t*>(m);
     m += b_bits;
     t->words = words;
+    t->lq = m;
+    m += b_lq;
     t->units = reinterpret_cast<unsigned long long*>(m);
     m += b_n8;
     t->ring = reinterpret_cast<int*>(m);
@@ -842,9 +850,7 @@ inline egt_status tile_prepare(egt_handle* h, TileArgs* t) {
     t->cloud_of = nullptr;
     t->npts = (int)n;
     cudaStream_t st = h->stream;
-    EGT_CUDA_TRY(cudaMemsetAsync(t->unit_bits, 0, b_bits, st));
-    EGT_CUDA_TRY(cudaMemsetAsync(tctr, 0, b_ctr, st));
-    EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrTileUnits, 0, 8 * sizeof(unsigned long long), st));
+    EGT_CUDA_TRY(cudaMemsetAsync(tctr, 0, b_ctr + b_bits, st));  // class counters and unit bits
     return EGT_OK;
 }
 
@@ -874,9 +880,7 @@ egt_status tile_kernel_launch(const KnnArgs& a, const TileArgs& t, cudaStream_t 
         std::lock_guard<std::mutex> lock(mu);
         waves[dev] = G;
     }
-    k_knn_tile<kBatch, S><<<G, kTileWarps * 32, smem, st>>>(a, t);
-    EGT_LAUNCH_CHECK();
-    return EGT_OK;
+    return launch_dependent(k_knn_tile<kBatch, S>, dim3(G), dim3(kTileWarps * 32), smem, st, a, t);
 }
 
 // kmax: the largest k among the queries the tile search takes.
@@ -884,13 +888,10 @@ template <bool kBatch>
 egt_status tile_launch(const KnnArgs& a, const TileArgs& t, int kmax, cudaStream_t st) {
     const unsigned T = 256;
     const int64_t npts = t.npts;
-    k_tile_assign<kBatch><<<(unsigned)((npts + T - 1) / T), T, 0, st>>>(a, t);
-    EGT_LAUNCH_CHECK();
+    EGT_TRY(launch_dependent(k_tile_assign<kBatch>, dim3((unsigned)((npts + T - 1) / T)), dim3(T), 0, st, a, t));
     const unsigned Gu = (unsigned)std::min<int64_t>(4096, (npts + T - 1) / T);
-    k_tile_count<kBatch><<<Gu, T, 0, st>>>(a, t);
-    EGT_LAUNCH_CHECK();
-    k_tile_gather<kBatch><<<Gu, T, 0, st>>>(a, t);
-    EGT_LAUNCH_CHECK();
+    EGT_TRY(launch_dependent(k_tile_count<kBatch>, dim3(Gu), dim3(T), 0, st, a, t));
+    EGT_TRY(launch_dependent(k_tile_gather<kBatch>, dim3(Gu), dim3(T), 0, st, a, t));
     return kmax <= kTileMaxK2 ? tile_kernel_launch<kBatch, 2>(a, t, st) : tile_kernel_launch<kBatch, 3>(a, t, st);
 }
 
