@@ -53,7 +53,7 @@ void free_handle(egt_handle* h) {
     F(h->d_counters); F(h->scratch.ptr);
     if (h->taubin_exec) cudaGraphExecDestroy(h->taubin_exec);
     F(h->m_perm); F(h->m_inv); F(h->m_p); F(h->m_pb); F(h->m_off); F(h->m_col);
-    F(h->t_uni); F(h->t_loc); F(h->t_nu); F(h->t_soff); F(h->tile_mem);
+    F(h->t_uni); F(h->t_loc); F(h->t_nu); F(h->t_soff); F(h->t_adj); F(h->tile_mem);
     cudaStreamSynchronize(h->stream);
     for (auto& e : h->ev)
         if (e) cudaEventDestroy(e);
@@ -530,6 +530,10 @@ egt_status egt_get_timings(egt_handle* h, egt_timings* t) {
     EGT_CUDA_TRY(cudaStreamSynchronize(h->stream));
     unsigned long long ctr[kCtrWords];
     EGT_CUDA_TRY(cudaMemcpy(ctr, h->d_counters, sizeof(ctr), cudaMemcpyDeviceToHost));
+    if (ctr[kCtrTaubinFail]) {
+        set_error("egt_taubin: a wait of the smoothing loop expired; the positions are NaN");
+        return EGT_ERR_TIMEOUT;
+    }
     h->tm.knn_ms = elapsed_ms(h->ev[2], h->ev[3]);
     h->tm.egt_ms = elapsed_ms(h->ev[4], h->ev[5]);
     h->tm.egt_kernel_ms = elapsed_ms(h->ev[4], h->ev[14]);

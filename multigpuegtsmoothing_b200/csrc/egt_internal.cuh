@@ -128,6 +128,7 @@ constexpr int kCtrNcells = 0;     // [0..7]  occupied cells per level (int in a 
 constexpr int kCtrExtents = 16;   // [16..18] six packed u32 min/max words
 constexpr int kCtrEgtTests = 24;    // EGT filter: ellipsoid tests of the last filter run
 constexpr int kCtrSpillTiles = 25;  // Taubin tiles that gather from global memory (too large to stage)
+constexpr int kCtrTaubinFail = 26;  // a wait of the resident Taubin loop expired
 constexpr int kCtrFlag = 27;      // generic loop flag
 constexpr int kCtrNormFallback = 28;  // normals re-solved in FP64
 constexpr int kCtrMsf = 29;       // spanning-forest edges
@@ -227,7 +228,9 @@ struct egt_handle {
     uint32_t* t_loc = nullptr;   // [tiles * 1792] CSR entries' slots, three 10-bit slots per word, sliced by warp
     int* t_nu = nullptr;         // [tiles] staged slot count, -1 = tile not staged
     int* t_soff = nullptr;       // [tiles * 9] slice offsets into t_loc, then the table size
-    int64_t t_tiles = 0;         // tiles the four tables above are sized for
+    uint32_t* t_adj = nullptr;   // small clouds: bits of the tiles each tile shares edges with (k_taubin_resident)
+    uint32_t taubin_tag = 0;     // tag of the next resident loop's first half-step
+    int64_t t_tiles = 0;         // tiles the tables above are sized for
     uint64_t csr_version = 0;    // bumped whenever the CSR is rebuilt
     uint64_t m_version = ~0ull;  // CSR version the Morton copy was built from
     // cached Taubin graph (2*iters half-steps) and the parameters it was built for

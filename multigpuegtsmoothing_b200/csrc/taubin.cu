@@ -21,6 +21,8 @@
 // Relabelling changes neither a row's neighbour order nor any value, so the
 // result is the same bit for bit.  Each half-step is a programmatic dependent
 // launch: its prologue (CSR tables only) overlaps the previous half-step.
+// Clouds whose tiles are all resident at once (592 tiles, 151K points) run the
+// loop in one launch instead (k_taubin_resident).
 #include <algorithm>
 #include <atomic>
 #include <climits>
@@ -167,6 +169,30 @@ __device__ __forceinline__ void tile_fetch(const TileRegs& r, const float4* __re
     cp_async_commit();
 }
 
+// One row's sums over its staged neighbours, in list order.  ls: the lane's
+// first slot word (entries 3g..3g+2 in word 32 g).  Three neighbours per step;
+// the next step's slot word is loaded before this step's positions are read,
+// off the critical path.
+__device__ __forceinline__ void tile_row(const float4* s_pos, const uint32_t* ls, int len, float4 p, float& cx,
+                                         float& cy, float& cz, float& sum) {
+    int e = 0;
+    uint32_t v = len > 0 ? ls[0] : 0u;
+#pragma unroll 1
+    for (; e + 3 <= len; e += 3) {
+        ls += 32;
+        const uint32_t vn = e + 3 < len ? *ls : v;
+        const float4 q0 = s_pos[v & 1023u], q1 = s_pos[(v >> 10) & 1023u], q2 = s_pos[v >> 20];
+        accumulate(p.x, p.y, p.z, q0, cx, cy, cz, sum);
+        accumulate(p.x, p.y, p.z, q1, cx, cy, cz, sum);
+        accumulate(p.x, p.y, p.z, q2, cx, cy, cz, sum);
+        v = vn;
+    }
+    if (e < len) {
+        accumulate(p.x, p.y, p.z, s_pos[v & 1023u], cx, cy, cz, sum);
+        if (e + 1 < len) accumulate(p.x, p.y, p.z, s_pos[(v >> 10) & 1023u], cx, cy, cz, sum);
+    }
+}
+
 // Staged half-step, persistent and double-buffered.  Every kTile-row tile
 // has its staged neighbour positions (t_uni: point index of each position
 // slot, precomputed once per CSR) and, per CSR entry, the 16-bit slot of its
@@ -227,25 +253,7 @@ __global__ void __launch_bounds__(kTile, 4) k_taubin_tiles(const float4* __restr
                 const float4* s_pos = reinterpret_cast<const float4*>(stage);
                 const uint32_t* ls =
                     reinterpret_cast<const uint32_t*>(stage + kUCap * sizeof(float4)) + cur.soff + lane;
-                const int len = cur.e1 - cur.e0;
-                // three neighbours per step; the next step's slot word is loaded
-                // before this step's positions are read, off the critical path
-                int e = 0;
-                uint32_t v = len > 0 ? ls[0] : 0u;
-#pragma unroll 1
-                for (; e + 3 <= len; e += 3) {
-                    ls += 32;
-                    const uint32_t vn = e + 3 < len ? *ls : v;
-                    const float4 q0 = s_pos[v & 1023u], q1 = s_pos[(v >> 10) & 1023u], q2 = s_pos[v >> 20];
-                    accumulate(p.x, p.y, p.z, q0, cx, cy, cz, sum);
-                    accumulate(p.x, p.y, p.z, q1, cx, cy, cz, sum);
-                    accumulate(p.x, p.y, p.z, q2, cx, cy, cz, sum);
-                    v = vn;
-                }
-                if (e < len) {
-                    accumulate(p.x, p.y, p.z, s_pos[v & 1023u], cx, cy, cz, sum);
-                    if (e + 1 < len) accumulate(p.x, p.y, p.z, s_pos[(v >> 10) & 1023u], cx, cy, cz, sum);
-                }
+                tile_row(s_pos, ls, cur.e1 - cur.e0, p, cx, cy, cz, sum);
             }
             pout[i] = finish(p, cx, cy, cz, sum, scale);
         }
@@ -257,6 +265,160 @@ __global__ void __launch_bounds__(kTile, 4) k_taubin_tiles(const float4* __restr
         i = tile * kTile + (int)threadIdx.x;
     }
     cp_async_wait<0>();
+}
+
+// 16 bytes as one relaxed access: a position and its tag are written and seen together.
+__device__ __forceinline__ void store_tagged(float4* p, float4 v) {
+    const unsigned long long lo = ((unsigned long long)__float_as_uint(v.y) << 32) | __float_as_uint(v.x);
+    const unsigned long long hi = ((unsigned long long)__float_as_uint(v.w) << 32) | __float_as_uint(v.z);
+    asm volatile("{ .reg .b128 q; mov.b128 q, {%1, %2}; st.relaxed.gpu.global.b128 [%0], q; }" ::"l"(p), "l"(lo),
+                 "l"(hi)
+                 : "memory");
+}
+__device__ __forceinline__ float4 load_tagged(const float4* p) {
+    unsigned long long lo, hi;
+    asm volatile("{ .reg .b128 q; ld.relaxed.gpu.global.b128 q, [%2]; mov.b128 {%0, %1}, q; }"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(p)
+                 : "memory");
+    return make_float4(__uint_as_float((uint32_t)lo), __uint_as_float((uint32_t)(lo >> 32)),
+                       __uint_as_float((uint32_t)hi), __uint_as_float((uint32_t)(hi >> 32)));
+}
+
+// All half-steps of a small cloud in one launch: every block keeps one tile's
+// slot table, point indices, row lengths and its rows' own positions on the
+// chip for the whole loop, and only positions of other tiles' points go
+// through L2, between two position buffers.  The w of a position is the number
+// of the half-step that wrote it (a tag; tag0 + step + 1), so a block simply
+// reads the positions it needs until they carry the tag of the last half-step:
+// no fence, flag or barrier lies between the store of a position and its use.
+//
+// A buffer is overwritten two half-steps later.  By then every tile that reads
+// it must have done so: a tile's rows carry a half-step's tag only after the
+// whole block has gathered that half-step's inputs, so it is enough that every
+// block sees the last half-step's tag in each tile that reads from it.  Tiles
+// it reads from itself are covered; s_dep lists the others (t_adj, symmetric),
+// of which it reads one row's tag.
+//
+// The blocks wait on one another, so the grid is launched cooperatively, one
+// block per tile, all resident.  A wait that does not end (kResidentPolls)
+// sets *fail and every block leaves; k_scatter_morton then writes NaN
+// positions, and the calls that read the handle's counters return
+// EGT_ERR_TIMEOUT.
+//
+// Bound: the latency of a half-step (store to L2, load from L2, the rows'
+// serial sums).  36K points 2.2 us per half-step, 131K-vertex mesh 2.1, 2,500
+// points 1.7.  A launch per half-step: 4.1, 5.3 and 3.5 us, and 1.1 ms of host
+// time to build and destroy a graph of 300 launches.  Flags per tile with a
+// fence and acquiring polls: 4.5, 9.5 and 2.2 us (the polls meet in a few
+// cache lines).
+constexpr int kResidentPolls = 1 << 22;
+constexpr int kResidentMaxTiles = 1024;  // entries of a block's list of reading tiles
+constexpr uint32_t kNoTag = 0xffffffffu;  // w of positions that no resident loop wrote
+constexpr size_t kResidentSmem = 2 * kUCap * sizeof(float4) + kSellWords * sizeof(uint32_t);
+
+__global__ void __launch_bounds__(kTile, 4) k_taubin_resident(
+    float4* buf_a, float4* buf_b, const int* __restrict__ off, const int* __restrict__ col,
+    const int* __restrict__ t_uni, const uint32_t* __restrict__ t_loc, const int* __restrict__ t_nu,
+    const int* __restrict__ t_soff, const uint32_t* __restrict__ t_adj, int adj_words, int n, int steps, float lambda,
+    float mu, uint32_t tag0, unsigned long long* __restrict__ fail) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint16_t s_dep[kResidentMaxTiles];
+    __shared__ uint32_t s_read[kResidentMaxTiles / 32];  // tiles this one reads from
+    __shared__ int16_t s_own[kTile];                     // staged slot of each of the tile's own rows (-1: none)
+    __shared__ int s_ndep;
+    const int tile = blockIdx.x, lane = threadIdx.x & 31;
+    float4* const s_pos = reinterpret_cast<float4*>(smem);  // two stages
+    uint32_t* const s_loc = reinterpret_cast<uint32_t*>(smem + 2 * kUCap * sizeof(float4));
+    const TileRegs r = tile_regs(off, t_uni, t_nu, t_soff, tile, n);
+    if (threadIdx.x == 0) s_ndep = 0;
+    if (threadIdx.x < kResidentMaxTiles / 32) s_read[threadIdx.x] = 0u;
+    s_own[threadIdx.x] = -1;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kUPer; u++) {
+        const int j = (int)threadIdx.x + u * kTile;
+        if (j < r.nu) {
+            const int from = r.uni[u] / kTile;
+            if (from == tile) s_own[r.uni[u] % kTile] = (int16_t)j;
+            else atomicOr(&s_read[from >> 5], 1u << (from & 31));
+        }
+    }
+    if (r.nu >= 0)
+        for (int v = threadIdx.x; v < (r.ssize + 3) >> 2; v += kTile)
+            cp_async16(s_loc + 4 * v, t_loc + (size_t)tile * kSellWords + 4 * v);
+    cp_async_commit();
+    __syncthreads();
+    for (int u = threadIdx.x; u < (int)gridDim.x; u += kTile)
+        if (u != tile && ((t_adj[(size_t)tile * adj_words + (u >> 5)] & ~s_read[u >> 5]) >> (u & 31) & 1u))
+            s_dep[atomicAdd(&s_ndep, 1)] = (uint16_t)u;
+    const int i = tile * kTile + (int)threadIdx.x;
+    float4 p = i < n ? buf_a[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    const int ndep = s_ndep, len = r.e1 - r.e0, own = s_own[threadIdx.x];
+    const uint32_t* const ls0 = s_loc + r.soff + lane;
+    cp_async_wait<0>();
+    int polls = 0;
+    bool lost = false;
+    // the position at q once it carries the tag
+    auto wait_for = [&](const float4* q, uint32_t tag) {
+        float4 v = load_tagged(q);
+        while (__float_as_uint(v.w) != tag && !lost) {
+            if (++polls >= kResidentPolls || ((polls & 1023) == 0 && *(volatile unsigned long long*)fail)) lost = true;
+            v = load_tagged(q);
+        }
+        return v;
+    };
+    for (int step = 0; step < steps; step++) {
+        const float4* pin = (step & 1) ? buf_b : buf_a;
+        float4* pout = (step & 1) ? buf_a : buf_b;
+        float4* stage = s_pos + (step & 1) * kUCap;
+        const uint32_t tag = tag0 + (uint32_t)step;
+        float cx = 0.0f, cy = 0.0f, cz = 0.0f, sum = 0.0f;
+        polls = 0;
+        if (step == 0) {  // the whole buffer is there
+#pragma unroll
+            for (int u = 0; u < kUPer; u++) {
+                const int j = (int)threadIdx.x + u * kTile;
+                if (j < r.nu) stage[j] = pin[r.uni[u]];
+            }
+        } else {
+            // all loads in flight at once, then each until it carries the tag;
+            // the tile's own rows are already staged
+            float4 v[kUPer];
+#pragma unroll
+            for (int u = 0; u < kUPer; u++) {
+                const int j = (int)threadIdx.x + u * kTile;
+                if (j < r.nu && r.uni[u] / kTile != tile) v[u] = load_tagged(pin + r.uni[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < kUPer; u++) {
+                const int j = (int)threadIdx.x + u * kTile;
+                if (j < r.nu && r.uni[u] / kTile != tile) {
+                    if (__float_as_uint(v[u].w) != tag) v[u] = wait_for(pin + r.uni[u], tag);
+                    stage[j] = v[u];
+                }
+            }
+            for (int d = threadIdx.x; d < ndep; d += kTile) wait_for(pin + s_dep[d] * kTile, tag);
+        }
+        if (r.nu < 0 && i < n) {  // tile too large to stage: its rows read their neighbours from the buffer
+            for (int e = r.e0; e < r.e1; e++) {
+                const float4* q = pin + __ldg(col + e);
+                accumulate(p.x, p.y, p.z, step ? wait_for(q, tag) : *q, cx, cy, cz, sum);
+            }
+        }
+        if (__syncthreads_or(lost)) {
+            if (threadIdx.x == 0) atomicExch(fail, 1ull);
+            break;
+        }
+        if (i < n) {
+            if (r.nu >= 0) tile_row(stage, ls0, len, p, cx, cy, cz, sum);
+            p = finish(p, cx, cy, cz, sum, (step & 1) ? mu : lambda);
+            p.w = __uint_as_float(step + 1 < steps ? tag + 1u : kNoTag);
+            store_tagged(pout + i, p);
+            if (own >= 0) s_pos[((step & 1) ^ 1) * kUCap + own] = p;
+        }
+    }
 }
 
 // Builds the tables of one tile (one block per tile): a block radix sort of
@@ -276,6 +438,7 @@ __global__ void __launch_bounds__(kBuildThreads) k_tile_build(const int* __restr
                                                               int n, int* __restrict__ t_uni,
                                                               uint32_t* __restrict__ t_loc, int* __restrict__ t_nu,
                                                               int* __restrict__ t_soff,
+                                                              uint32_t* __restrict__ t_adj, int adj_words,
                                                               unsigned long long* __restrict__ spilled) {
     using Sort = cub::BlockRadixSort<int, kBuildThreads, kBuildItems>;
     using Scan = cub::BlockScan<int, kBuildThreads>;
@@ -290,13 +453,23 @@ __global__ void __launch_bounds__(kBuildThreads) k_tile_build(const int* __restr
     __shared__ int s_soff[kSoffWords];
     __shared__ int s_nu;
     const int tile = blockIdx.x;
+    // tile u shares an edge with this one (t_adj: symmetric bits, for k_taubin_resident)
+    auto joined = [&](int u) {
+        atomicOr(&t_adj[(size_t)tile * adj_words + (u >> 5)], 1u << (u & 31));
+        atomicOr(&t_adj[(size_t)u * adj_words + (tile >> 5)], 1u << (tile & 31));
+    };
+    auto spill = [&]() {  // not staged: its neighbours are not listed, so it counts as joined to every tile
+        if (threadIdx.x == 0) { t_nu[tile] = -1; atomicAdd(spilled, 1ull); }
+        if (t_adj)
+            for (int u = threadIdx.x; u < (int)gridDim.x; u += kBuildThreads) joined(u);
+    };
     const int base = tile * kTile;
     const int last = min(base + kTile, n);
     const int rows = last - base;
     const int e_lo = off[base], e_hi = off[last];
     const int cnt = e_hi - e_lo;
     if (cnt > kTileCap) {
-        if (threadIdx.x == 0) { t_nu[tile] = -1; atomicAdd(spilled, 1ull); }
+        spill();
         return;
     }
     int keys[kBuildItems];
@@ -331,7 +504,7 @@ __global__ void __launch_bounds__(kBuildThreads) k_tile_build(const int* __restr
     __syncthreads();
     const int nu = s_nu;
     if (nu > kUCap) {
-        if (threadIdx.x == 0) { t_nu[tile] = -1; atomicAdd(spilled, 1ull); }
+        spill();
         return;
     }
     for (int i = threadIdx.x; i < cnt; i += kBuildThreads) {
@@ -354,10 +527,14 @@ __global__ void __launch_bounds__(kBuildThreads) k_tile_build(const int* __restr
     }
     __syncthreads();
     if (s_soff[kSlices] > kSellWords) {
-        if (threadIdx.x == 0) { t_nu[tile] = -1; atomicAdd(spilled, 1ull); }
+        spill();
         return;
     }
-    for (int u = threadIdx.x; u < nu; u += kBuildThreads) t_uni[(size_t)tile * kUCap + u] = sm.uniq[u];
+    for (int u = threadIdx.x; u < nu; u += kBuildThreads) {
+        t_uni[(size_t)tile * kUCap + u] = sm.uniq[u];
+        // the distinct neighbours are sorted: one entry per tile
+        if (t_adj && (u == 0 || sm.uniq[u] / kTile != sm.uniq[u - 1] / kTile)) joined(sm.uniq[u] / kTile);
+    }
     const int ssize = s_soff[kSlices];
     for (int x = threadIdx.x; x < ssize; x += kBuildThreads) {
         int w = 0;
@@ -447,16 +624,23 @@ __global__ void k_morton_cols(const int* __restrict__ perm, const int* __restric
 __global__ void k_gather_morton(const float4* __restrict__ p4, const int* __restrict__ perm, int n,
                                 float4* __restrict__ mp) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) mp[i] = p4[perm[i]];
+    if (i >= n) return;
+    float4 v = p4[perm[i]];
+    v.w = __uint_as_float(kNoTag);
+    mp[i] = v;
 }
 
+// failed: a resident loop gave up (k_taubin_resident); its positions are no result.
 __global__ void k_scatter_morton(const float4* __restrict__ mp, const int* __restrict__ perm, int n,
                                  float4* __restrict__ p4, float* __restrict__ x, float* __restrict__ y,
-                                 float* __restrict__ z) {
+                                 float* __restrict__ z, const uint32_t* __restrict__ cell0,
+                                 const unsigned long long* __restrict__ failed) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float4 v = mp[i];
+    float4 v = mp[i];
+    if (*failed) v.x = v.y = v.z = __int_as_float(0x7fffffff);
     const int s = perm[i];
+    v.w = __uint_as_float(cell0[s]);  // as the grid build stores it
     p4[s] = v;
     x[s] = v.x; y[s] = v.y; z[s] = v.z;
 }
@@ -502,6 +686,8 @@ static egt_status staged_launch(egt_handle* h, const float4* pin, float4* pout, 
     return EGT_OK;
 }
 
+static int adj_words(int64_t tiles) { return (int)((tiles + 31) / 32); }
+
 // Builds the Morton-order copy of the CSR (when the CSR changed) and gathers
 // the current positions into Morton order.
 static egt_status morton_prepare(egt_handle* h) {
@@ -513,6 +699,7 @@ static egt_status morton_prepare(egt_handle* h) {
         EGT_CUDA_TRY(dev_alloc(h, &h->m_inv, sizeof(int) * n));
         EGT_CUDA_TRY(dev_alloc(h, &h->m_p, sizeof(float4) * n));
         EGT_CUDA_TRY(dev_alloc(h, &h->m_pb, sizeof(float4) * n));
+        EGT_CUDA_TRY(cudaMemsetAsync(h->m_pb, 0xff, sizeof(float4) * n, st));  // no tags (k_taubin_resident)
         EGT_CUDA_TRY(dev_alloc(h, &h->m_off, sizeof(int) * (n + 1)));
     }
     if (h->m_version != h->csr_version) {
@@ -582,11 +769,16 @@ static egt_status morton_prepare(egt_handle* h) {
             EGT_CUDA_TRY(dev_alloc(h, &h->t_loc, sizeof(uint32_t) * kSellWords * tiles));
             EGT_CUDA_TRY(dev_alloc(h, &h->t_nu, sizeof(int) * tiles));
             EGT_CUDA_TRY(dev_alloc(h, &h->t_soff, sizeof(int) * kSoffWords * tiles));
+            if (h->t_adj) dev_free(h, h->t_adj);
+            h->t_adj = nullptr;
+            if (tiles <= kResidentMaxTiles) EGT_CUDA_TRY(dev_alloc(h, &h->t_adj, sizeof(uint32_t) * tiles * adj_words(tiles)));
             h->t_tiles = tiles;
         }
+        if (h->t_adj) EGT_CUDA_TRY(cudaMemsetAsync(h->t_adj, 0, sizeof(uint32_t) * tiles * adj_words(tiles), st));
         EGT_CUDA_TRY(cudaMemsetAsync(h->d_counters + kCtrSpillTiles, 0, sizeof(unsigned long long), st));
         k_tile_build<<<(unsigned)tiles, kBuildThreads, 0, st>>>(h->m_off, h->m_col, n, h->t_uni, h->t_loc, h->t_nu,
-                                                                 h->t_soff, h->d_counters + kCtrSpillTiles);
+                                                                 h->t_soff, h->t_adj, adj_words(tiles),
+                                                                 h->d_counters + kCtrSpillTiles);
         EGT_LAUNCH_CHECK();
         h->tm.taubin_tiles = tiles;
         cudaFreeAsync(kin, st);
@@ -597,6 +789,37 @@ static egt_status morton_prepare(egt_handle* h) {
     }
     k_gather_morton<<<G, 256, 0, st>>>(h->p4, h->m_perm, n, h->m_p);
     EGT_LAUNCH_CHECK();
+    return EGT_OK;
+}
+
+// The whole loop over a cloud whose tiles are all resident at once.
+static egt_status resident_loop(egt_handle* h, int iters, float lambda, float mu, cudaStream_t st) {
+    const int n = (int)h->n, tiles = (n + kTile - 1) / kTile;
+    for (int left = iters; left > 0;) {  // long loops in several launches: the tags stay far from wrapping
+        const int part = std::min(left, 1 << 24);
+        if (h->taubin_tag > 0xf0000000u) {  // (kNoTag and tags of long ago are never waited for)
+            h->taubin_tag = 0;
+            EGT_CUDA_TRY(cudaMemsetAsync(h->m_pb, 0xff, sizeof(float4) * (size_t)n, st));
+        }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)tiles);
+        cfg.blockDim = dim3(kTile);
+        cfg.dynamicSmemBytes = kResidentSmem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        EGT_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_taubin_resident, h->m_p, h->m_pb, (const int*)h->m_off,
+                                        (const int*)h->m_col, (const int*)h->t_uni, (const uint32_t*)h->t_loc,
+                                        (const int*)h->t_nu, (const int*)h->t_soff, (const uint32_t*)h->t_adj,
+                                        adj_words(tiles), n, 2 * part, lambda, mu, h->taubin_tag,
+                                        h->d_counters + kCtrTaubinFail));
+        EGT_LAUNCH_CHECK();
+        h->taubin_tag += 2u * (uint32_t)part;
+        left -= part;
+    }
     return EGT_OK;
 }
 
@@ -612,7 +835,7 @@ egt_status run_taubin(egt_handle* h, int iters, float lambda, float mu) {
         // function attributes are per device: set them once on each, and size
         // the persistent grid from the occupancy they allow
         static std::atomic<uint64_t> attr_set{0};
-        static std::atomic<unsigned> wave[64];
+        static std::atomic<unsigned> wave[64], resident[64];  // blocks of one resident wave
         int dev = 0;
         EGT_CUDA_TRY(cudaGetDevice(&dev));
         if (!(attr_set.load() >> (dev & 63) & 1)) {
@@ -626,9 +849,24 @@ egt_status run_taubin(egt_handle* h, int iters, float lambda, float mu) {
             EGT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
             EGT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_taubin_tiles, kTile, kPipeSmem));
             wave[dev & 63].store((unsigned)std::max(1, sms * std::max(per, 1)));
+            EGT_CUDA_TRY(cudaFuncSetAttribute(k_taubin_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)kResidentSmem));
+            EGT_CUDA_TRY(cudaFuncSetAttribute(k_taubin_resident, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                              (int)cudaSharedmemCarveoutMaxShared));
+            EGT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_taubin_resident, kTile, kResidentSmem));
+            resident[dev & 63].store((unsigned)(sms * per));
             attr_set.fetch_or(uint64_t(1) << (dev & 63));
         }
         const unsigned blocks = wave[dev & 63].load();
+        const int tiles = (n + kTile - 1) / kTile;
+        if (h->taubin_mode == 0 && h->t_adj && tiles <= (int)resident[dev & 63].load()) {
+            EGT_TRY(resident_loop(h, iters, lambda, mu, st));
+            k_scatter_morton<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(h->m_p, h->m_perm, n, h->p4, h->x, h->y,
+                                                                           h->z, h->cell0, h->d_counters + kCtrTaubinFail);
+            EGT_LAUNCH_CHECK();
+            EGT_CUDA_TRY(cudaEventRecord(h->ev[7], st));
+            return EGT_OK;
+        }
         // every buffer the captured launches name
         const void* key[8] = {h->m_p, h->m_pb, h->t_uni, h->t_loc, h->t_nu, h->t_soff, h->m_off, h->m_col};
         const bool reuse = h->taubin_exec && h->taubin_iters == iters && h->taubin_lambda == lambda &&
@@ -680,7 +918,7 @@ egt_status run_taubin(egt_handle* h, int iters, float lambda, float mu) {
         }
         EGT_CUDA_TRY(cudaGraphLaunch(h->taubin_exec, st));
         k_scatter_morton<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(h->m_p, h->m_perm, n, h->p4, h->x, h->y,
-                                                                       h->z);
+                                                                       h->z, h->cell0, h->d_counters + kCtrTaubinFail);
         EGT_LAUNCH_CHECK();
     } else {
         k_split_soa<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(h->p4, n, h->x, h->y, h->z);
