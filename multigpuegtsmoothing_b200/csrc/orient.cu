@@ -24,6 +24,9 @@
 // its raw sign there).  Component sign votes (Normal_CUDA.cu:517-711) only act
 // on list edges that join different trees; the trees are the connected
 // components of the list graph, so there are none to act on.
+//
+// The host waits once per few rounds (kRoundsPerSync): every kernel of a round
+// reads its sizes from the device, and ends at once when nothing is left.
 #include <cub/cub.cuh>
 #include <numeric>
 #include <vector>
@@ -34,23 +37,113 @@ namespace {
 
 constexpr unsigned long long kNone = ~0ull;
 
-// Warp-aggregated counter increment: one atomic per warp.  Every lane of the
-// warp must call it (pred false for lanes without an item).
-__device__ __forceinline__ void warp_count(unsigned long long* ctr, bool pred) {
-    const unsigned b = __ballot_sync(0xffffffffu, pred);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(ctr, (unsigned long long)__popc(b));
+constexpr int kTB = 256;  // threads per block
+
+// Block-aggregated counter increment.  Every thread of the block must call it
+// (pred false for threads without an item).
+__device__ __forceinline__ void block_count(unsigned long long* ctr, bool pred) {
+    const int c = __syncthreads_count(pred);
+    if (threadIdx.x == 0 && c) atomicAdd(ctr, (unsigned long long)c);
 }
 
-__global__ void k_edge_keys(const int* __restrict__ off, const int* __restrict__ col, int n, int bits,
-                            unsigned long long* __restrict__ key) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const unsigned long long sentinel = (1ull << (2 * bits)) - 1ull;
-    for (int e = off[i]; e < off[i + 1]; e++) {
+// ---- the undirected edges of the lists, in key order ----
+// Every edge {u, v}, u < v, belongs to the bucket of u.  Row u's own entries
+// above u go there directly; an entry u of a row v > u only if row u does not
+// list v (most do, so few entries need an atomic).  A bucket is then ordered
+// by v (rank by counting, buckets are short) and repeated entries dropped, which
+// puts the edges in (u, v) order: the reference's key order, without sorting
+// 64-bit keys (1M points, 16M list entries: 1.03 ms with a radix sort).
+
+constexpr int kRowLanes = 16;  // lanes per row
+
+// keep[e]: 1 = bucket of its own row, 2 = bucket of the other end.  own[i]:
+// entries of kind 1; cnt[u]: entries of bucket u (zero before).
+__global__ void __launch_bounds__(kTB) k_bucket_count(const int* __restrict__ off, const int* __restrict__ col, int n,
+                                                      unsigned char* __restrict__ keep, int* __restrict__ own,
+                                                      int* __restrict__ cnt) {
+    const int i = (int)((blockIdx.x * (int64_t)kTB + threadIdx.x) / kRowLanes);
+    const int l = threadIdx.x & (kRowLanes - 1);
+    const int e0 = i < n ? off[i] : 0, e1 = i < n ? off[i + 1] : 0;
+    int mine = 0;
+    for (int e = e0 + l; e < e1; e += kRowLanes) {
         const int m = col[e];
-        const unsigned u = (unsigned)min(i, m), v = (unsigned)max(i, m);
-        key[e] = (u == v) ? sentinel : (((unsigned long long)u << bits) | v);
+        unsigned char kind = 0;
+        if (m > i) {
+            kind = 1;
+            mine++;
+        } else if (m < i) {
+            const int f0 = off[m], f1 = off[m + 1];
+            kind = 2;
+            for (int f = f0; f < f1; f++)
+                if (col[f] == i) { kind = 0; break; }
+            if (kind) atomicAdd(&cnt[m], 1);
+        }
+        keep[e] = kind;
     }
+#pragma unroll
+    for (int o = kRowLanes / 2; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+    if (l == 0 && i < n) {
+        own[i] = mine;
+        if (mine) atomicAdd(&cnt[i], mine);
+    }
+}
+
+// Fills the buckets (boff: their starts).  own[u] becomes bucket u's next free
+// place after its own row's entries.
+__global__ void __launch_bounds__(kTB) k_bucket_fill(const int* __restrict__ off, const int* __restrict__ col, int n,
+                                                     int bits, const unsigned char* __restrict__ keep,
+                                                     const int* __restrict__ boff, int* __restrict__ own,
+                                                     unsigned long long* __restrict__ key) {
+    const int i = (int)((blockIdx.x * (int64_t)kTB + threadIdx.x) / kRowLanes);
+    const int l = threadIdx.x & (kRowLanes - 1);
+    const int e0 = i < n ? off[i] : 0, e1 = i < n ? off[i + 1] : 0;
+    const unsigned gmask = 0xffffu << (threadIdx.x & 16);
+    int at = i < n ? boff[i] : 0;
+    const int rounds = (e1 - e0 + kRowLanes - 1) / kRowLanes;
+    for (int r = 0; r < rounds; r++) {  // uniform over the row's lanes
+        const int e = e0 + r * kRowLanes + l;
+        const int kind = e < e1 ? keep[e] : 0;
+        const unsigned b = __ballot_sync(gmask, kind == 1) & gmask;
+        if (kind) {
+            const int m = col[e];
+            if (kind == 1) {
+                key[at + __popc(b & ((1u << (threadIdx.x & 31)) - 1u))] = ((unsigned long long)i << bits) | (unsigned)m;
+            } else {
+                key[boff[m] + atomicAdd(&own[m], 1)] = ((unsigned long long)m << bits) | (unsigned)i;
+            }
+        }
+        at += __popc(b);
+    }
+}
+
+// Orders every bucket and gives its edges their places: ukey[p] the edge at
+// place p, act[p] its order key (weight bits, p) -- p grows with the vertex key,
+// so this is the reference's (weight, key) order -- and sgn[p] the sign of its
+// dot product.  The place of a repeated entry stays empty (kNone).
+__global__ void __launch_bounds__(kTB) k_bucket_edges(const unsigned long long* __restrict__ key,
+                                                      const int* __restrict__ boff, int n, int bits,
+                                                      const float* __restrict__ nrm,
+                                                      unsigned long long* __restrict__ ukey,
+                                                      unsigned long long* __restrict__ act,
+                                                      signed char* __restrict__ sgn) {
+    const int64_t e = blockIdx.x * (int64_t)kTB + threadIdx.x;
+    if (e >= boff[n]) return;
+    const unsigned long long k = key[e];
+    const int u = (int)(k >> bits), v = (int)(k & ((1ull << bits) - 1ull));
+    const int b0 = boff[u], b1 = boff[u + 1];
+    int p = b0;
+    bool again = false;
+    for (int f = b0; f < b1; f++) {
+        const unsigned long long o = key[f];
+        p += (o < k || (o == k && f < e)) ? 1 : 0;
+        again |= o == k && f < e;
+    }
+    ukey[p] = k;
+    if (again) { act[p] = kNone; return; }
+    const float d = fs_dot3(nrm[u], nrm[n + u], nrm[2 * (size_t)n + u], nrm[v], nrm[n + v], nrm[2 * (size_t)n + v]);
+    const float w = fmaxf(0.0f, __fsub_rn(1.0f, fabsf(d)));
+    act[p] = ((unsigned long long)__float_as_uint(w) << 32) | (unsigned)p;
+    sgn[p] = d < 0.0f ? -1 : 1;
 }
 
 // 1 for the first copy of each edge key in the sorted array (self-loop
@@ -63,58 +156,102 @@ __global__ void k_first_copy(const unsigned long long* __restrict__ key, int64_t
     flag[e] = (k != (1ull << (2 * bits)) - 1ull) && (e == 0 || key[e - 1] != k);
 }
 
-// Edge e's order key (weight bits, e) -- e is the rank of the edge's vertex
-// key, so this is the reference's (weight, key) order -- and its sign.
-__global__ void k_edge_init(const unsigned long long* __restrict__ ukey, int E, int bits,
-                            const float* __restrict__ nrm, int n, unsigned long long* __restrict__ ckey,
-                            signed char* __restrict__ sgn) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    const unsigned long long k = ukey[e];
-    const int u = (int)(k >> bits), v = (int)(k & ((1ull << bits) - 1ull));
-    const float d = fs_dot3(nrm[u], nrm[n + u], nrm[2 * (size_t)n + u], nrm[v], nrm[n + v], nrm[2 * (size_t)n + v]);
-    const float w = fmaxf(0.0f, __fsub_rn(1.0f, fabsf(d)));
-    ckey[e] = ((unsigned long long)__float_as_uint(w) << 32) | (unsigned)e;
-    sgn[e] = d < 0.0f ? -1 : 1;
-}
+// State of a forest computation on the device.
+struct ForestState {
+    int live[2];               // edges of the two edge lists
+    unsigned long long linked;  // links of the last round
+};
 
-__global__ void k_init_comp(int n, int* __restrict__ comp, signed char* __restrict__ sig) {
+__global__ void k_init_comp(int n, const int* __restrict__ edges, int max_edges, int* __restrict__ comp,
+                            signed char* __restrict__ sig, unsigned long long* __restrict__ best,
+                            ForestState* __restrict__ fs) {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v == 0) {
+        fs->live[0] = edges ? *edges : max_edges;
+        fs->live[1] = 0;
+        fs->linked = 0;
+    }
     if (v >= n) return;
     comp[v] = v;
     sig[v] = 1;
+    best[v] = kNone;
 }
 
-// Lightest live edge of every component.  act: order keys of the edges that
-// joined two components at the start of the round (*live of them).
-__global__ void k_select(const unsigned long long* __restrict__ act, const int* __restrict__ live,
-                         const unsigned long long* __restrict__ ukey, int bits, const int* __restrict__ comp,
-                         unsigned long long* __restrict__ best) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= *live) return;
-    const unsigned long long c = act[i];
-    const unsigned long long k = ukey[c & 0xffffffffull];
-    const int u = (int)(k >> bits), v = (int)(k & ((1ull << bits) - 1ull));
-    const int cu = comp[u], cv = comp[v];
-    if (cu == cv) return;
-    atomicMin(&best[cu], c);
-    atomicMin(&best[cv], c);
+// Lightest live edge of every component.  in: the edges that joined two
+// components when the last round began; those that still do are copied to out,
+// so dead edges are read once more and no pass of its own drops them.  Most
+// edges are not lighter than what their component has seen, which a read
+// tells without an atomic (1M points, 9M edges, first round: 245 us with two
+// atomics per edge).  One count atomic per block.
+constexpr int kSelItems = 8;
+__global__ void __launch_bounds__(kTB) k_select(const unsigned long long* __restrict__ in,
+                                                unsigned long long* __restrict__ out, int side,
+                                                const unsigned long long* __restrict__ ukey, int bits,
+                                                const int* __restrict__ comp, unsigned long long* best,
+                                                ForestState* __restrict__ fs) {
+    __shared__ int s_cnt[kTB / 32], s_base;
+    const int live = fs->live[side];
+    if (blockIdx.x == 0 && threadIdx.x == 0) fs->linked = 0;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int64_t i0 = (int64_t)blockIdx.x * kTB * kSelItems; i0 < live; i0 += (int64_t)gridDim.x * kTB * kSelItems) {
+        unsigned long long c[kSelItems];
+        unsigned mask[kSelItems];
+        int cnt = 0;
+#pragma unroll
+        for (int j = 0; j < kSelItems; j++) {
+            const int64_t i = i0 + j * kTB + threadIdx.x;
+            c[j] = i < live ? in[i] : kNone;
+        }
+#pragma unroll
+        for (int j = 0; j < kSelItems; j++) {
+            bool joins = false;
+            if (c[j] != kNone) {
+                const unsigned long long k = ukey[c[j] & 0xffffffffull];
+                const int cu = comp[(int)(k >> bits)], cv = comp[(int)(k & ((1ull << bits) - 1ull))];
+                joins = cu != cv;
+                if (joins) {
+                    if (c[j] < *(volatile unsigned long long*)&best[cu]) atomicMin(&best[cu], c[j]);
+                    if (c[j] < *(volatile unsigned long long*)&best[cv]) atomicMin(&best[cv], c[j]);
+                }
+            }
+            mask[j] = __ballot_sync(0xffffffffu, joins);
+            cnt += __popc(mask[j]);
+        }
+        if (lane == 0) s_cnt[w] = cnt;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int total = 0;
+            for (int u = 0; u < kTB / 32; u++) { const int t = s_cnt[u]; s_cnt[u] = total; total += t; }
+            s_base = total ? atomicAdd(&fs->live[side ^ 1], total) : 0;
+        }
+        __syncthreads();
+        int at = s_base + s_cnt[w];
+#pragma unroll
+        for (int j = 0; j < kSelItems; j++) {
+            if ((mask[j] >> lane) & 1u) out[at + __popc(mask[j] & ((1u << lane) - 1u))] = c[j];
+            at += __popc(mask[j]);
+        }
+        __syncthreads();
+    }
 }
 
-// Hooks every component to the one across its lightest edge.  A pair that
-// chose each other links only the larger representative.  Counts the links
-// (= forest edges added) into ctr[kCtrFlag] and ctr[kCtrMsf].
-__global__ void k_hook(const unsigned long long* __restrict__ ukey, const signed char* __restrict__ sgn, int n,
-                       int bits, const int* __restrict__ comp, const signed char* __restrict__ sig,
-                       const unsigned long long* __restrict__ best, int* __restrict__ link,
-                       signed char* __restrict__ lpar, unsigned long long* __restrict__ ctr,
-                       unsigned char* __restrict__ msf) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+// Hooks every component to the one across its lightest edge: link[c] = (that
+// component << 1) | (1 when the signs across differ); a root links to itself.
+// A pair that chose each other links only the larger representative.  Counts
+// the links (= forest edges added).  first (optional): the round's choices.
+__global__ void __launch_bounds__(kTB) k_hook(const unsigned long long* __restrict__ ukey,
+                                              const signed char* __restrict__ sgn, int n, int bits, int side,
+                                              const int* __restrict__ comp, const signed char* __restrict__ sig,
+                                              const unsigned long long* __restrict__ best, unsigned* __restrict__ link,
+                                              unsigned long long* __restrict__ first, ForestState* __restrict__ fs,
+                                              unsigned long long* __restrict__ ctr, unsigned char* __restrict__ msf) {
+    const int c = blockIdx.x * kTB + threadIdx.x;
     bool linked = false;
+    if (c == 0) fs->live[side] = 0;  // the list this round read: the next round's output
     if (c < n) {
-        link[c] = c;
-        lpar[c] = 1;
         const unsigned long long b = comp[c] == c ? best[c] : kNone;
+        if (first) first[c] = b;
+        unsigned to = (unsigned)c << 1;
         if (b != kNone) {
             const int e = (int)(b & 0xffffffffull);
             const unsigned long long k = ukey[e];
@@ -123,50 +260,55 @@ __global__ void k_hook(const unsigned long long* __restrict__ ukey, const signed
             const int y = x == u ? v : u;
             const int c2 = comp[y];
             if (!(best[c2] == b && c < c2)) {  // mutual choice: the smaller representative stays a root
-                link[c] = c2;
-                lpar[c] = (signed char)(sig[x] * sgn[e] * sig[y]);
+                to = ((unsigned)c2 << 1) | (sig[x] * sgn[e] * sig[y] < 0 ? 1u : 0u);
                 linked = true;
                 if (msf) msf[e] = 1;
             }
         }
+        link[c] = to;
     }
-    warp_count(&ctr[kCtrFlag], linked);
-    warp_count(&ctr[kCtrMsf], linked);
+    const int t = __syncthreads_count(linked);
+    if (threadIdx.x == 0 && t) {
+        atomicAdd(&fs->linked, (unsigned long long)t);
+        atomicAdd(&ctr[kCtrMsf], (unsigned long long)t);
+    }
 }
 
-__global__ void k_jump(const int* __restrict__ link, const signed char* __restrict__ lpar, int n,
-                       int* __restrict__ link2, signed char* __restrict__ lpar2, unsigned long long* __restrict__ ctr) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    bool moved = false;
-    if (c < n) {
-        const int l = link[c];
-        const int ll = link[l];
-        moved = l != ll;
-        link2[c] = ll;
-        lpar2[c] = moved ? (signed char)(lpar[c] * lpar[l]) : lpar[c];
+// Shortens the link chains in place: a component follows the links it finds,
+// which other threads shorten meanwhile (target and sign are one word, and
+// every word is a true path of its component, old or new).
+constexpr int kJumps = 32;
+__global__ void __launch_bounds__(kTB) k_jump(unsigned* link, int n, const int* __restrict__ comp,
+                                              const ForestState* __restrict__ fs) {
+    const int c = blockIdx.x * kTB + threadIdx.x;
+    if (c >= n || fs->linked == 0 || comp[c] != c) return;
+    unsigned w = link[c];
+    for (int it = 0; it < kJumps; it++) {
+        const unsigned l = w >> 1;
+        const unsigned wl = *(volatile unsigned*)&link[l];
+        if ((wl >> 1) == l) break;
+        w = (wl & ~1u) | ((w ^ wl) & 1u);
+        *(volatile unsigned*)&link[c] = w;
     }
-    warp_count(&ctr[kCtrFlag], moved);
 }
 
-__global__ void k_relabel(int n, const int* __restrict__ link, const signed char* __restrict__ lpar,
-                          int* __restrict__ comp, signed char* __restrict__ sig) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n) return;
-    const int c = comp[v];
-    comp[v] = link[c];
-    sig[v] = (signed char)(sig[v] * lpar[c]);
-}
-
-// An edge that still joins two components.
-struct JoinsTwo {
-    const unsigned long long* ukey;
-    const int* comp;
-    int bits;
-    __device__ bool operator()(unsigned long long c) const {
-        const unsigned long long k = ukey[c & 0xffffffffull];
-        return comp[(int)(k >> bits)] != comp[(int)(k & ((1ull << bits) - 1ull))];
+// Every vertex to its component's root (the rest of a chain that k_jump did
+// not finish is followed here).
+__global__ void __launch_bounds__(kTB) k_relabel(int n, const unsigned* __restrict__ link, int* __restrict__ comp,
+                                                 signed char* __restrict__ sig, unsigned long long* __restrict__ best,
+                                                 const ForestState* __restrict__ fs) {
+    const int v = blockIdx.x * kTB + threadIdx.x;
+    if (v >= n || fs->linked == 0) return;
+    unsigned w = link[comp[v]];
+    for (;;) {
+        const unsigned wl = link[w >> 1];
+        if ((wl >> 1) == (w >> 1)) break;
+        w = (wl & ~1u) | ((w ^ wl) & 1u);
     }
-};
+    comp[v] = (int)(w >> 1);
+    if (w & 1u) sig[v] = (signed char)-sig[v];
+    best[v] = kNone;
+}
 
 // Lightest edge of every tree.  It is the lightest edge at one of its ends, so
 // it is the minimum of the first round's choices (first) over the tree's
@@ -207,7 +349,7 @@ __global__ void k_apply(int n, int bits, const int* __restrict__ comp, const sig
             }
         }
     }
-    warp_count(&ctr[kCtrComps], root);
+    block_count(&ctr[kCtrComps], root);
 }
 
 // ---- orient_kruskal (MST.cpp:399-423): the reference's CPU orienter ----
@@ -304,93 +446,75 @@ __global__ void k_kr_apply(int n, const int* __restrict__ comp, const int* __res
     }
 }
 
-__global__ void k_set_int(int* p, int v) { *p = v; }
-
 // Device buffers of one spanning-forest computation over n vertices.
 struct Forest {
     int* comp = nullptr;
-    int* link = nullptr;
-    int* link2 = nullptr;
+    unsigned* link = nullptr;
     signed char* sig = nullptr;
-    signed char* lpar = nullptr;
-    signed char* lpar2 = nullptr;
     unsigned long long* best = nullptr;
     unsigned long long* first = nullptr;
+    ForestState* state = nullptr;
 
     cudaError_t alloc(int n, cudaStream_t st) {
         cudaError_t e = cudaSuccess;
         auto A = [&](auto** p, size_t bytes) {
             if (e == cudaSuccess) e = cudaMallocAsync((void**)p, bytes, st);
         };
-        A(&comp, sizeof(int) * n); A(&link, sizeof(int) * n); A(&link2, sizeof(int) * n);
-        A(&sig, n); A(&lpar, n); A(&lpar2, n);
+        A(&comp, sizeof(int) * n); A(&link, sizeof(unsigned) * n); A(&sig, n);
         A(&best, sizeof(unsigned long long) * n); A(&first, sizeof(unsigned long long) * n);
+        A(&state, sizeof(ForestState));
         return e;
     }
     void release(cudaStream_t st) {
-        for (void* p : {(void*)comp, (void*)link, (void*)link2, (void*)sig, (void*)lpar, (void*)lpar2, (void*)best,
-                        (void*)first})
+        for (void* p : {(void*)comp, (void*)link, (void*)sig, (void*)best, (void*)first, (void*)state})
             if (p) cudaFreeAsync(p, st);
     }
 };
 
+constexpr int kRoundsPerSync = 4;
+
 // Borůvka minimum spanning forest with sign parity.  act[0..E): order keys
-// (rank << 32 | edge), the low half indexing ukey (u << bits | v) and sgn
-// (+-1); the order keys are compacted in place as edges fall inside one
-// component.  On return f.comp[v] is v's component representative, f.sig[v]
-// the product of the edge signs on the forest path from the representative to
-// v, and f.first[v] the order key of v's lightest edge.  msf (optional):
-// msf[edge] = 1 for every forest edge.  ctr: device counters (kCtrFlag and
-// kCtrMsf are used).  tmp / t_live: scratch for cub::DeviceSelect::If.
+// (rank << 32 | edge; kNone: no edge), the low half indexing ukey (u << bits |
+// v) and sgn (+-1); edges (optional): their number on the device, at most E.
+// act and act2 (E entries) take turns as the list of edges between components.
+// On return f.comp[v] is v's component representative, f.sig[v] the product of
+// the edge signs on the forest path from the representative to v, and
+// f.first[v] the order key of v's lightest edge.  msf (optional): msf[edge] =
+// 1 for every forest edge.  ctr: device counters (kCtrMsf is used).
 egt_status spanning_forest(int n, int E, int bits, const unsigned long long* ukey, unsigned long long* act,
-                           const signed char* sgn, int* d_num, void* tmp, size_t t_live,
+                           unsigned long long* act2, const int* edges, const signed char* sgn,
                            unsigned long long* ctr, Forest& f, unsigned char* msf, cudaStream_t st) {
-    const unsigned TB = 256;
-    auto G = [&](int64_t m) { return (unsigned)((m + TB - 1) / TB); };
-    k_set_int<<<1, 1, 0, st>>>(d_num, E);
-    EGT_LAUNCH_CHECK();
-    k_init_comp<<<G(n), TB, 0, st>>>(n, f.comp, f.sig);
+    auto G = [&](int64_t m) { return (unsigned)((m + kTB - 1) / kTB); };
+    k_init_comp<<<G(n), kTB, 0, st>>>(n, edges, E, f.comp, f.sig, f.best, f.state);
     EGT_LAUNCH_CHECK();
     if (E == 0) {  // every vertex is its own component
         EGT_CUDA_TRY(cudaMemsetAsync(f.first, 0xff, sizeof(unsigned long long) * n, st));
         return EGT_OK;
     }
-    JoinsTwo live_op{ukey, f.comp, bits};
-    // each round at least halves the non-trivial components; *d_num counts
-    // the live edges at the head of act
-    int live = E;  // *d_num, read back once per round (an upper bound until then)
+    // each round at least halves the non-trivial components
+    int64_t live = E;  // upper bound of the list's length
+    unsigned long long* list[2] = {act, act2};
     for (int round = 0;; round++) {
         if (round > 64) { set_error("orientation: spanning forest did not converge"); return EGT_ERR_CAP_EXCEEDED; }
-        EGT_CUDA_TRY(cudaMemsetAsync(f.best, 0xff, sizeof(unsigned long long) * n, st));
-        EGT_CUDA_TRY(cudaMemsetAsync(ctr + kCtrFlag, 0, sizeof(unsigned long long), st));
-        k_select<<<G(live), TB, 0, st>>>(act, d_num, ukey, bits, f.comp, f.best);
+        const int side = round & 1;
+        const unsigned gs = (unsigned)std::max<int64_t>(
+            1, std::min<int64_t>((live + kTB * kSelItems - 1) / (kTB * kSelItems), 148 * 8));
+        k_select<<<gs, kTB, 0, st>>>(list[side], list[side ^ 1], side, ukey, bits, f.comp, f.best, f.state);
         EGT_LAUNCH_CHECK();
-        if (round == 0)  // every vertex's lightest edge: the tree roots come from these
-            EGT_CUDA_TRY(cudaMemcpyAsync(f.first, f.best, sizeof(unsigned long long) * n, cudaMemcpyDeviceToDevice, st));
-        k_hook<<<G(n), TB, 0, st>>>(ukey, sgn, n, bits, f.comp, f.sig, f.best, f.link, f.lpar, ctr, msf);
+        k_hook<<<G(n), kTB, 0, st>>>(ukey, sgn, n, bits, side, f.comp, f.sig, f.best, f.link,
+                                     round == 0 ? f.first : nullptr, f.state, ctr, msf);
         EGT_LAUNCH_CHECK();
-        unsigned long long any = 0;
-        EGT_CUDA_TRY(cudaMemcpyAsync(&any, ctr + kCtrFlag, sizeof(any), cudaMemcpyDeviceToHost, st));
-        EGT_CUDA_TRY(cudaMemcpyAsync(&live, d_num, sizeof(int), cudaMemcpyDeviceToHost, st));
-        EGT_CUDA_TRY(cudaStreamSynchronize(st));  // live is now exact: the compaction below reads it
-        if (!any) break;
-        // pointer jumping over the hook forest, composing the sign parities
-        for (int it = 0;; it++) {
-            if (it > 64) { set_error("orientation: pointer jumping did not converge"); return EGT_ERR_CAP_EXCEEDED; }
-            EGT_CUDA_TRY(cudaMemsetAsync(ctr + kCtrFlag, 0, sizeof(unsigned long long), st));
-            k_jump<<<G(n), TB, 0, st>>>(f.link, f.lpar, n, f.link2, f.lpar2, ctr);
-            EGT_LAUNCH_CHECK();
-            std::swap(f.link, f.link2);
-            std::swap(f.lpar, f.lpar2);
-            unsigned long long ch = 0;
-            EGT_CUDA_TRY(cudaMemcpyAsync(&ch, ctr + kCtrFlag, sizeof(ch), cudaMemcpyDeviceToHost, st));
+        k_jump<<<G(n), kTB, 0, st>>>(f.link, n, f.comp, f.state);
+        EGT_LAUNCH_CHECK();
+        k_relabel<<<G(n), kTB, 0, st>>>(n, f.link, f.comp, f.sig, f.best, f.state);
+        EGT_LAUNCH_CHECK();
+        if (round % kRoundsPerSync == kRoundsPerSync - 1) {
+            ForestState s;
+            EGT_CUDA_TRY(cudaMemcpyAsync(&s, f.state, sizeof(s), cudaMemcpyDeviceToHost, st));
             EGT_CUDA_TRY(cudaStreamSynchronize(st));
-            if (!ch) break;
+            if (s.linked == 0) break;
+            live = s.live[side ^ 1];
         }
-        k_relabel<<<G(n), TB, 0, st>>>(n, f.link, f.lpar, f.comp, f.sig);
-        EGT_LAUNCH_CHECK();
-        // drop the edges that now lie inside one component
-        EGT_CUDA_TRY(cub::DeviceSelect::If(tmp, t_live, act, d_num, live, live_op, st));
     }
     return EGT_OK;
 }
@@ -410,60 +534,48 @@ egt_status run_orient(egt_handle* h) {
     }
     int bits = 1;
     while ((1ll << bits) < (int64_t)n) bits++;
-    const unsigned TB = 256;
-    auto G = [&](int64_t m) { return (unsigned)((m + TB - 1) / TB); };
-    // 1. undirected edge keys u*2^bits+v (u < v), sorted (key order = the
-    // reference's hash order), first copies kept in place.  The two halves of
-    // the sort's double buffer are the only edge-sized buffers: after the
-    // sort one holds the edges, the other their order keys.
-    unsigned long long *bufA = nullptr, *bufB = nullptr;
-    unsigned char* flag = nullptr;
-    int* d_num = nullptr;
-    EGT_CUDA_TRY(cudaMallocAsync((void**)&bufA, sizeof(unsigned long long) * nnz, st));
-    EGT_CUDA_TRY(cudaMallocAsync((void**)&bufB, sizeof(unsigned long long) * nnz, st));
-    EGT_CUDA_TRY(cudaMallocAsync((void**)&flag, nnz, st));
-    EGT_CUDA_TRY(cudaMallocAsync((void**)&d_num, sizeof(int), st));
-    k_edge_keys<<<G(n), TB, 0, st>>>(h->csr_off, h->csr_col, n, bits, bufA);
+    auto G = [&](int64_t m) { return (unsigned)((m + kTB - 1) / kTB); };
+    // 1. undirected edges in key order, with their order keys and signs
+    size_t t_scan = 0;
+    EGT_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, t_scan, (int*)nullptr, (int*)nullptr, n + 1, st));
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t a = at; at += (bytes + 255) & ~(size_t)255; return a; };
+    const size_t o_key = take(sizeof(unsigned long long) * nnz), o_ukey = take(sizeof(unsigned long long) * nnz),
+                 o_act = take(sizeof(unsigned long long) * nnz), o_sgn = take(nnz), o_keep = take(nnz),
+                 o_cnt = take(sizeof(int) * (n + 1)), o_boff = take(sizeof(int) * (n + 1)),
+                 o_own = take(sizeof(int) * n), o_scan = take(t_scan);
+    char* m = nullptr;
+    EGT_CUDA_TRY(cudaMallocAsync((void**)&m, at, st));
+    auto* key = reinterpret_cast<unsigned long long*>(m + o_key);
+    auto* ukey = reinterpret_cast<unsigned long long*>(m + o_ukey);
+    auto* act = reinterpret_cast<unsigned long long*>(m + o_act);
+    auto* sgn = reinterpret_cast<signed char*>(m + o_sgn);
+    auto* keep = reinterpret_cast<unsigned char*>(m + o_keep);
+    auto* cnt = reinterpret_cast<int*>(m + o_cnt);
+    auto* boff = reinterpret_cast<int*>(m + o_boff);
+    auto* own = reinterpret_cast<int*>(m + o_own);
+    EGT_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int) * (n + 1), st));
+    k_bucket_count<<<G((int64_t)n * kRowLanes), kTB, 0, st>>>(h->csr_off, h->csr_col, n, keep, own, cnt);
     EGT_LAUNCH_CHECK();
-    cub::DoubleBuffer<unsigned long long> keys(bufA, bufB);
-    size_t t_sort = 0, t_flag = 0, t_live = 0;
-    EGT_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, t_sort, keys, (int)nnz, 0, 2 * bits, st));
-    EGT_CUDA_TRY(cub::DeviceSelect::Flagged(nullptr, t_flag, bufA, flag, d_num, (int)nnz, st));
-    JoinsTwo live_op{nullptr, nullptr, bits};
-    EGT_CUDA_TRY(cub::DeviceSelect::If(nullptr, t_live, bufA, d_num, (int)nnz, live_op, st));
-    void* tmp = nullptr;
-    EGT_TRY(scratch_reserve(h, std::max(std::max(t_sort, t_flag), t_live), &tmp));
-    EGT_CUDA_TRY(cub::DeviceRadixSort::SortKeys(tmp, t_sort, keys, (int)nnz, 0, 2 * bits, st));
-    unsigned long long* ukey = keys.Current();
-    unsigned long long* act = keys.Alternate();
-    k_first_copy<<<G(nnz), TB, 0, st>>>(ukey, nnz, bits, flag);
+    EGT_CUDA_TRY(cub::DeviceScan::ExclusiveSum(m + o_scan, t_scan, cnt, boff, n + 1, st));
+    k_bucket_fill<<<G((int64_t)n * kRowLanes), kTB, 0, st>>>(h->csr_off, h->csr_col, n, bits, keep, boff, own, key);
     EGT_LAUNCH_CHECK();
-    EGT_CUDA_TRY(cub::DeviceSelect::Flagged(tmp, t_flag, ukey, flag, d_num, (int)nnz, st));
-    int E = 0;
-    EGT_CUDA_TRY(cudaMemcpyAsync(&E, d_num, sizeof(int), cudaMemcpyDeviceToHost, st));
-    EGT_CUDA_TRY(cudaStreamSynchronize(st));
-    // ukey now holds the E unique edges in ascending key order
-    signed char* sgn = nullptr;
-    EGT_CUDA_TRY(cudaMallocAsync((void**)&sgn, std::max(E, 1), st));
+    k_bucket_edges<<<G(nnz), kTB, 0, st>>>(key, boff, n, bits, h->nrm, ukey, act, sgn);
+    EGT_LAUNCH_CHECK();
+    // 2. Borůvka rounds (the unordered edges' buffer is free again)
     Forest f;
     EGT_CUDA_TRY(f.alloc(n, st));
-    egt_status status = EGT_OK;
-    if (E > 0) {
-        k_edge_init<<<G(E), TB, 0, st>>>(ukey, E, bits, h->nrm, n, act, sgn);
+    egt_status status =
+        spanning_forest(n, (int)nnz, bits, ukey, act, key, boff + n, sgn, h->d_counters, f, nullptr, st);
+    if (status == EGT_OK) {
+        // 3. roots (first vertex of each tree's lightest edge) and signs
+        EGT_CUDA_TRY(cudaMemsetAsync(f.best, 0xff, sizeof(unsigned long long) * n, st));
+        k_roots<<<G(n), kTB, 0, st>>>(n, f.comp, f.first, f.best);
         EGT_LAUNCH_CHECK();
-        // 2. Borůvka rounds
-        status = spanning_forest(n, E, bits, ukey, act, sgn, d_num, tmp, t_live, h->d_counters, f, nullptr, st);
-        if (status == EGT_OK) {
-            // 3. roots (first vertex of each tree's lightest edge) and signs
-            EGT_CUDA_TRY(cudaMemsetAsync(f.best, 0xff, sizeof(unsigned long long) * n, st));
-            k_roots<<<G(n), TB, 0, st>>>(n, f.comp, f.first, f.best);
-            EGT_LAUNCH_CHECK();
-            k_apply<<<G(n), TB, 0, st>>>(n, bits, f.comp, f.sig, f.best, ukey, h->nrm, h->d_counters);
-            EGT_LAUNCH_CHECK();
-        }
+        k_apply<<<G(n), kTB, 0, st>>>(n, bits, f.comp, f.sig, f.best, ukey, h->nrm, h->d_counters);
+        EGT_LAUNCH_CHECK();
     }
-    cudaFreeAsync(bufA, st); cudaFreeAsync(bufB, st); cudaFreeAsync(flag, st); cudaFreeAsync(d_num, st);
-    cudaFreeAsync(sgn, st);
+    cudaFreeAsync(m, st);
     f.release(st);
     EGT_CUDA_TRY(cudaEventRecord(h->ev[11], st));
     return status;
@@ -566,13 +678,11 @@ egt_status run_orient_kruskal(const int* knn, float* nrm, int n, int k, int k_us
     EGT_CUDA_TRY(D(&f1, E));
     EGT_CUDA_TRY(D(&f2, E));
     EGT_CUDA_TRY(D(&f3, E));
-    size_t t_pairs = 0, t_live = 0, t_sel = 0;
+    size_t t_pairs = 0, t_sel = 0;
     EGT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, t_pairs, wkey, wkey2, eidx, order, E, 0, 64, st));
-    JoinsTwo probe{nullptr, nullptr, bits};
-    EGT_CUDA_TRY(cub::DeviceSelect::If(nullptr, t_live, act, d_num, E, probe, st));
     EGT_CUDA_TRY(cub::DeviceSelect::Flagged(nullptr, t_sel, vkey, f1, sel, d_num, E, st));
     void* tmp2 = nullptr;
-    EGT_CUDA_TRY(D(&tmp2, std::max(std::max(t_pairs, t_live), t_sel)));
+    EGT_CUDA_TRY(D(&tmp2, std::max(t_pairs, t_sel)));
     EGT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp2, t_pairs, wkey, wkey2, eidx, order, E, 0, 64, st));
     k_kr_rank<<<G(E), TB, 0, st>>>(order, E, act);
     EGT_LAUNCH_CHECK();
@@ -585,7 +695,8 @@ egt_status run_orient_kruskal(const int* knn, float* nrm, int n, int k, int k_us
         ~ForestReleaser() { f.release(st); }
     } fr{f, st};
     EGT_CUDA_TRY(f.alloc(n, st));
-    EGT_TRY(spanning_forest(n, E, bits, ukey, act, sgn, d_num, tmp2, t_live, ctr, f, msf, st));
+    // (the second edge list: the unsorted weights are no longer needed)
+    EGT_TRY(spanning_forest(n, E, bits, ukey, act, wkey, nullptr, sgn, ctr, f, msf, st));
     // forest edges in Kruskal order, and the zero-dot ones among them
     k_kr_forest_lists<<<G(E), TB, 0, st>>>(order, E, ukey, msf, zero, vkey, okey, f1, f2, f3);
     EGT_LAUNCH_CHECK();
@@ -650,7 +761,7 @@ egt_status run_orient_kruskal(const int* knn, float* nrm, int n, int k, int k_us
         EGT_CUDA_TRY(cudaMemcpyAsync(&e2, d_num, sizeof(int), cudaMemcpyDeviceToHost, st));
         EGT_CUDA_TRY(cudaStreamSynchronize(st));
         EGT_CUDA_TRY(g.alloc(n, st));
-        EGT_TRY(spanning_forest(n, e2, bits, ukey, sel, sgn, d_num, tmp2, t_live, ctr, g, nullptr, st));
+        EGT_TRY(spanning_forest(n, e2, bits, ukey, sel, wkey, nullptr, sgn, ctr, g, nullptr, st));
         std::vector<int> part((size_t)n);
         EGT_CUDA_TRY(cudaMemcpyAsync(part.data(), g.comp, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
         EGT_CUDA_TRY(cudaStreamSynchronize(st));
