@@ -633,7 +633,8 @@ egt_status knn_batch(egt_batch* b) {
     bool tile = b->cfg.knn_mode == EGT_KNN_TILE;
     if (tile) {
         tile = false;
-        for (int c = 0; c < b->count; c++) tile |= b->k[c] >= kTileMinK && b->k[c] <= kTileMaxK;
+        // (the batch's points share the launches: their total decides)
+        for (int c = 0; c < b->count; c++) tile |= tile_takes(b->N, b->k[c]);
     }
     if (tile) {
         if (kk + 1 <= 32) EGT_TRY(knn_batch_tile<1>(b, st));

@@ -77,6 +77,13 @@ __device__ __forceinline__ float fs_dist3(float ax, float ay, float az, float bx
     float dx = __fsub_rn(ax, bx), dy = __fsub_rn(ay, by), dz = __fsub_rn(az, bz);
     return __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
 }
+// fs_dist3 of one point against two (packed FP32: the same roundings in each
+// half, half the instructions).  (nx, ny, nz): the two points' coordinates,
+// negated; a + (-b) is a - b bit for bit.
+__device__ __forceinline__ float2 fs_dist3x2(float2 ax, float2 ay, float2 az, float2 nx, float2 ny, float2 nz) {
+    const float2 dx = __fadd2_rn(ax, nx), dy = __fadd2_rn(ay, ny), dz = __fadd2_rn(az, nz);
+    return __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
+}
 __device__ __forceinline__ float fs_sq3(float x, float y, float z) {
     return __fmaf_rn(z, z, __fmaf_rn(x, x, __fmul_rn(y, y)));
 }
@@ -200,6 +207,7 @@ struct egt_handle {
     uint8_t* pclass = nullptr;   // [n] proposed class per query
     const egt_proposal* proposal = nullptr;  // attached for knn_mode == EGT_KNN_LEARNED
     bool last_knn_learned = false;
+    bool knn_untiled = false;    // EGT_KNN_TILE ran the ring search for every query (a small cloud)
     void* tile_mem = nullptr;    // cell-tile kNN: query levels, unit bits, units, leftover queries
     size_t tile_bytes = 0;
     int* csr_off = nullptr;      // [n+1]

@@ -866,7 +866,9 @@ egt_status run_knn(egt_handle* h, int k) {
     EGT_TRY(knn_prepare(h, k, &a));
     EGT_TRY(reset_knn_counters(h));
     EGT_CUDA_TRY(cudaEventRecord(h->ev[2], st));
-    if (h->cfg.knn_mode == EGT_KNN_TILE && k >= kTileMinK && k <= kTileMaxK) EGT_TRY(tile_search(h, a, st));
+    const bool tile = h->cfg.knn_mode == EGT_KNN_TILE;
+    h->knn_untiled = tile && k >= kTileLowK && k <= kTileMaxK && !tile_takes(h->n, k);
+    if (tile && tile_takes(h->n, k)) EGT_TRY(tile_search(h, a, st));
     else EGT_TRY(knn_search(a, h->cfg.knn_mode == EGT_KNN_SELECT, st));
     EGT_CUDA_TRY(cudaEventRecord(h->ev[3], st));
     return EGT_OK;
@@ -927,6 +929,7 @@ __global__ void k_rows_original(const int* __restrict__ lists, const int* __rest
 // them.
 egt_status run_knn_host(egt_handle* h, int k, int* host) {
     cudaStream_t st = h->stream;
+    h->knn_untiled = false;
     KnnArgs a;
     EGT_TRY(knn_prepare(h, k, &a));
     const int n = (int)h->n;

@@ -12,15 +12,19 @@
 // of its lanes at once:
 //
 //   pass 1  each lane buckets its candidate distances (64 buckets, 8 per
-//           octave of d^2 from (h/4)^2 to (4h)^2, h the level's cell side)
-//           and finds the bucket b* holding its (k+1)-th smallest; the half
-//           records the smallest bucket of each group of steps;
-//   pass 2  each lane keeps the block positions (16 bits) of buckets <= b*
-//           (at most tile_cap) in bucket order (offsets from pass 1's counts),
-//           visiting only the step groups whose smallest bucket is at most
-//           the half's largest b*; the kept distances are computed again into
-//           the spent bucket space and the list is insertion-sorted (only
-//           candidates of one bucket are out of order).
+//           octave of d^2, placed around the k-th distance that the block's
+//           population suggests) and finds the bucket b* holding its (k+1)-th
+//           smallest; the half records the smallest bucket of each group of
+//           steps;
+//   pass 2  each lane appends the candidates of buckets <= b* (at most
+//           kKeep), visiting only the step groups whose smallest bucket is at
+//           most the half's largest b*.  A kept candidate is one word: the
+//           upper 19 bits of its distance's place in the bucket range, and its
+//           13-bit position in the block;
+//   sort    the words go through a sorting network in registers, the lanes side
+//           by side.  Words whose 19 bits agree (distances below the bucket
+//           range, and a chance pair in a hundred queries) are put in order by
+//           their distances, computed again.
 //
 // The result is accepted only when it provably equals the ring search's list
 // (the conditions of the proposal-driven box search, knn.cu): the k+1
@@ -39,6 +43,7 @@
 #pragma once
 #include <map>
 #include <mutex>
+#include <utility>
 #include "knn_search.cuh"
 #include "proposal.cuh"
 
@@ -47,16 +52,35 @@ namespace {
 
 constexpr int kTileWarps = 1;    // warps per block (one: blocks pack the SM's shared memory tightly)
 constexpr int kTileBins = 64;    // distance buckets per query: 8 per octave of d^2, (h/4)^2 to (4h)^2
-// S: list registers of the in-kernel ring search (k+1 <= 32 S); it also sets
-// the candidates kept per query (the buckets up to b*, the query included).
-template <int S>
-constexpr int tile_cap() { return S <= 2 ? 64 : 96; }
-constexpr int kTileMinK = 16;    // smaller k: the ring search (measured faster there)
+// Forms of the search by k: list registers S of the in-kernel ring search
+// (k+1 <= 32 S) and words kept per query, the query included (kKeep): k+2 and
+// the rest of the last bucket, which is 9 % of the count below it on a surface.
+// kWarps: warps per SM.  20 leave 96 registers a thread (4M points, k = 40: 9.23
+// ms of kNN with 16 warps, 8.37 with 20, 8.69 with 23); the longest form needs
+// more registers for its sorting network.
+struct TileForm1 { static constexpr int S = 1, kKeep = 32, kMaxK = 22, kWarps = 20; };
+struct TileForm2 { static constexpr int S = 2, kKeep = 56, kMaxK = 40, kWarps = 20; };
+struct TileForm3 { static constexpr int S = 3, kKeep = 80, kMaxK = 64, kWarps = 16; };
+constexpr int kTilePosBits = 13;  // block positions (kTileMaxBlock)
+constexpr int kTileMaxUnsorted = 16;  // points below the bucket range a query may have (more: the ring search)
+// Smallest k and cloud the tile search takes.  Below kTileMinPoints points its
+// chain of launches and its long batches cost more than the ring search of
+// every query (k = 40: 8K points 151 against 53 us, 36K 217 against 168; 72K 274
+// against 304); k of 8 to 15 pays from kTileMinPointsLowK points (k = 10: 36K
+// points 131 against 136 us, 72K 150 against 248, 1M 1.95 against 2.60 ms).
+constexpr int kTileMinK = 8;
+constexpr int kTileLowK = 16;
+constexpr int64_t kTileMinPoints = 50000;
+constexpr int64_t kTileMinPointsLowK = 65536;
 constexpr int kTileMaxK = 64;    // largest k the cell-tile search takes
-constexpr int kTileMaxK2 = 40;   // largest k of the narrower form (S = 2, 64 kept candidates)
-constexpr int kTileAlpha = 6;    // block population that selects a level, in units of k+1 (measured on
-                                 // 4M superquadrics at k = 40, with the sparse rule below: 5 to 7 within
-                                 // 2 %, 4 and 8 slower)
+inline bool tile_takes(int64_t n, int k) {
+    return k >= kTileMinK && k <= kTileMaxK && n >= (k < kTileLowK ? kTileMinPointsLowK : kTileMinPoints);
+}
+constexpr int kTileAlpha = 6;    // block population that selects a level, in units of k+1 (4M
+                                 // superquadrics, k = 40: 8.37 ms; 5: 8.69; 4: 9.56, more rows uncertified)
+constexpr int kTileEff = 24;     // smaller k select a block as if k were this: blocks of fewer points hold
+                                 // fewer queries than lanes (1M points: k = 10 2.34 -> 1.96 ms, k = 16
+                                 // 2.42 -> 2.30; 40 in its place: 2.02 and 2.33)
 constexpr int kTileSparse = 2;       // a finer block below (k+1)/kTileSparse points: the ring search (measured
                                       // on 4M superquadrics at k = 40: (k+1)/2 and 0.6(k+1) best, 0.75(k+1)
                                       // 8 % slower, 0.45(k+1) and below 15 % slower: its long searches return)
@@ -111,23 +135,20 @@ __device__ __forceinline__ void unit_parts(unsigned long long code, int& c, int&
     ci = (int)(code & 0xffffffffu);
 }
 
-// Shared memory of one warp (both halves).
-// Rows of the bucket space: the buckets, then the kept candidates' distances
-// (one row each, up to tile_cap).
-template <int S>
-constexpr int tile_rows() { return kTileBins > tile_cap<S>() ? kTileBins : tile_cap<S>(); }
+constexpr int kTileStage = 3 * 16;
 
-template <int S>
+// Shared memory of one warp (both halves).
+// Rows of the bucket space: the buckets, then the kept words (one row each).
+template <typename Form>
+constexpr int tile_rows() { return kTileBins > Form::kKeep ? kTileBins : Form::kKeep; }
+
+template <typename Form>
 constexpr size_t tile_warp_bytes() {
-    return (size_t)tile_rows<S>() * 32 * 4         // bucket counts, offsets, then kept distances [row][lane]
-           + (size_t)tile_cap<S>() * 32 * 2        // kept candidates' block positions [slot][lane]
-           + 2 * 16 * 16                           // staged candidates per half (x, y, z, point)
+    return (size_t)tile_rows<Form>() * 32 * 4      // bucket counts, then kept words [row][lane]
+           + 2 * kTileStage * 4                    // staged candidates per half: x, y, z of 16, negated
            + 2 * 2 * 16 * 4;                       // per half: range sequence scratch at unit set-up,
                                                    // then the step groups' smallest buckets
 }
-
-// Kept-candidate slot s of lane `lane` (16-bit entries: two lanes per bank word).
-__device__ __forceinline__ int tile_slot(int s, int lane) { return s * 32 + lane; }
 
 // Index of level cell (cx, cy, cz) in the level's cell arrays (-1: empty).
 __device__ __forceinline__ int cell_index(const LevelDev& L, int cx, int cy, int cz) {
@@ -182,7 +203,7 @@ __global__ void __launch_bounds__(256) k_tile_assign(KnnArgs a, TileArgs t) {
     int lsel = -1, ci = -1;
     // thres > 4 exceeds every squared distance of the unit cube: all admitted
     if (in && A.k >= kTileMinK && A.k <= kTileMaxK && A.np->thres > 4.0f) {
-        const int thr = kTileAlpha * (A.k + 1), sparse = (A.k + 1) / kTileSparse;
+        const int thr = kTileAlpha * (max(A.k, kTileEff) + 1), sparse = (A.k + 1) / kTileSparse;
         const uint32_t c0 = __float_as_uint(A.p4[q].w);
         const int cx0 = c0 & 1023u, cy0 = (c0 >> 10) & 1023u, cz0 = (c0 >> 20) & 1023u;
         // Population of the block of level l around the query's cell; the
@@ -396,15 +417,86 @@ __device__ __forceinline__ int seq_index16(const RangeSeq& q, int base, int hl, 
     return order ? __ldg(order + pos) : pos;
 }
 
-__device__ __forceinline__ uint32_t tile_bin(float d, uint32_t lo) {
-    return min((max(__float_as_uint(d), lo) - lo) >> 20, (uint32_t)(kTileBins - 1));
+// Distance buckets: an eighth of an octave of d^2 each, so the upper bits of
+// the float (sign, exponent, three bits of the mantissa) number them; `first`
+// is the number of bucket 0.  tile_clamp puts a distance into the range of the
+// kTileBins buckets (NaN into the last: never kept).
+constexpr int kTileShift = 20;
+__device__ __forceinline__ float tile_clamp(float d, uint32_t first) {
+    return fmaxf(fminf(d, __uint_as_float((first + kTileBins - 1) << kTileShift)),
+                 __uint_as_float(first << kTileShift));
 }
+// Shared-memory address of a clamped distance's bucket; base: that of number 0
+// for the lane (bucket rows are 32 words).
+__device__ __forceinline__ uint32_t tile_addr(float clamped, uint32_t base) {
+    return base + ((__float_as_uint(clamped) >> kTileShift) << 7);
+}
+__device__ __forceinline__ void shared_inc(uint32_t addr) {
+    asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(addr) : "memory");
+}
+// Squared distances of the lane's query to the half's 16 staged candidates.
+__device__ __forceinline__ void tile_distances(const float* stage, float4 pq, float d[16]) {
+    const float2 qx = make_float2(pq.x, pq.x), qy = make_float2(pq.y, pq.y), qz = make_float2(pq.z, pq.z);
+#pragma unroll
+    for (int j = 0; j < 16; j += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(stage + j);
+        const float4 y = *reinterpret_cast<const float4*>(stage + 16 + j);
+        const float4 z = *reinterpret_cast<const float4*>(stage + 32 + j);
+        const float2 a = fs_dist3x2(qx, qy, qz, make_float2(x.x, x.y), make_float2(y.x, y.y), make_float2(z.x, z.y));
+        const float2 b = fs_dist3x2(qx, qy, qz, make_float2(x.z, x.w), make_float2(y.z, y.w), make_float2(z.z, z.w));
+        d[j] = a.x;
+        d[j + 1] = a.y;
+        d[j + 2] = b.x;
+        d[j + 3] = b.y;
+    }
+}
+
+// Batcher's merge exchange (Knuth, The Art of Computer Programming, vol. 3,
+// algorithm 5.2.2M) for N elements: 32: 191 comparators, 56: 462, 80: 842.
+template <int N>
+struct SortNet {
+    static constexpr int count() {
+        int c = 0;
+        for (int p = 1; p < N; p *= 2)
+            for (int k = p; k >= 1; k /= 2)
+                for (int j = k % p; j + k < N; j += 2 * k)
+                    for (int i = 0; i < k && i + j + k < N; i++)
+                        if ((i + j) / (2 * p) == (i + j + k) / (2 * p)) c++;
+        return c;
+    }
+    struct Table { unsigned char a[count()], b[count()]; };
+    static constexpr Table make() {
+        Table t{};
+        int c = 0;
+        for (int p = 1; p < N; p *= 2)
+            for (int k = p; k >= 1; k /= 2)
+                for (int j = k % p; j + k < N; j += 2 * k)
+                    for (int i = 0; i < k && i + j + k < N; i++)
+                        if ((i + j) / (2 * p) == (i + j + k) / (2 * p)) {
+                            t.a[c] = (unsigned char)(i + j);
+                            t.b[c++] = (unsigned char)(i + j + k);
+                        }
+        return t;
+    }
+    static constexpr Table table = make();
+    template <int A, int B>
+    static __device__ __forceinline__ void exchange(uint32_t (&v)[N]) {
+        const uint32_t lo = min(v[A], v[B]), hi = max(v[A], v[B]);
+        v[A] = lo;
+        v[B] = hi;
+    }
+    template <size_t... C>
+    static __device__ __forceinline__ void run(uint32_t (&v)[N], std::index_sequence<C...>) {
+        (exchange<table.a[C], table.b[C]>(v), ...);
+    }
+    static __device__ __forceinline__ void sort(uint32_t (&v)[N]) { run(v, std::make_index_sequence<count()>()); }
+};
 
 // State of one half-warp's current unit (uniform within the half).
 struct TileUnit {
     RangeSeq seq;
     const int* order;
-    uint32_t lo;   // float bits of the lower edge of bucket 1 less one bucket
+    uint32_t first;  // number of bucket 0 (tile_clamp)
     int l;         // level; -1 = no unit
     // the block's ranges r < seq.m: pref[r] = inclusive prefix end of range r
     // (INT_MAX past the last), adj[r] = its start less the positions before it
@@ -426,10 +518,10 @@ __device__ __forceinline__ int tile_point(int pos, const TileUnit& U) {
 // Streams both halves' blocks through their staging buffers, 16 candidates
 // per half at a time, calling f(s) for step s: the half's staged candidates
 // are the block positions 16 s .. 16 s + 15 (padding past a block's end lies
-// far away with index -1).
+// far away).
 template <typename F>
 __device__ __forceinline__ void tile_stream16(const TileUnit& U, bool live, int steps, const float4* __restrict__ p4,
-                                              float4* chunk, int hl, int hf, F&& f) {
+                                              float* stage, int hl, int hf, F&& f) {
     const float4 far = make_float4(1e18f, 1e18f, 1e18f, 0.f);
     // software pipeline: the point index of step s+2 and the position of
     // step s+1 are in flight while step s is compared
@@ -439,7 +531,9 @@ __device__ __forceinline__ void tile_stream16(const TileUnit& U, bool live, int 
     float4 vB = pB >= 0 ? __ldg(p4 + pB) : far;
     for (int s = 0; s < steps; s++) {
         __syncwarp();
-        chunk[hl] = make_float4(vB.x, vB.y, vB.z, __int_as_float(pB));
+        stage[hl] = -vB.x;
+        stage[16 + hl] = -vB.y;
+        stage[32 + hl] = -vB.z;
         __syncwarp();
         pB = pA;
         vB = pB >= 0 ? __ldg(p4 + pB) : far;
@@ -455,7 +549,7 @@ __device__ __forceinline__ void tile_stream16(const TileUnit& U, bool live, int 
 // until both halves are done; a half that is done stages padding.
 template <typename N, typename F>
 __device__ __forceinline__ void tile_stream16_seq(const TileUnit& U, int s0, int end, N&& nxt,
-                                                  const float4* __restrict__ p4, float4* chunk, int hl, int hf,
+                                                  const float4* __restrict__ p4, float* stage, int hl, int hf,
                                                   F&& f) {
     const float4 far = make_float4(1e18f, 1e18f, 1e18f, 0.f);
     int s1 = nxt(s0), s2 = nxt(s1);
@@ -466,7 +560,9 @@ __device__ __forceinline__ void tile_stream16_seq(const TileUnit& U, int s0, int
     float4 vB = pB >= 0 ? __ldg(p4 + pB) : far;
     while (__any_sync(0xffffffffu, s0 < end)) {
         __syncwarp();
-        chunk[hl] = make_float4(vB.x, vB.y, vB.z, __int_as_float(pB));
+        stage[hl] = -vB.x;
+        stage[16 + hl] = -vB.y;
+        stage[32 + hl] = -vB.z;
         __syncwarp();
         pB = pA;
         vB = pB >= 0 ? __ldg(p4 + pB) : far;
@@ -512,19 +608,32 @@ __device__ __forceinline__ void tile_unit_setup(const KnnArgs& a, const NormPara
             if (t < 8) U.pref[t] = end;
             if (in) before = end;
         }
-        // buckets: 8 per octave of d^2, bucket 0 below (h/4)^2 and 1/8 octave,
-        // bucket kTileBins-1 from 16 h^2 up
+        // Buckets: 8 per octave of d^2, eight octaves.  The block's population on
+        // a surface through it (9 h^2) puts the k-th distance at
+        // (k+1) 9 h^2 / (pi pop): four octaves of buckets lie above that (three:
+        // 2.4 % of 4M superquadric rows uncertified instead of 1.7 %), four
+        // below, where about one point in 16 of the k is nearer than bucket 0.
         const float h = __fmul_rn(__fsub_rn(np.b, np.a), (float)(1 << l) * (1.0f / 1024.0f));
-        U.lo = __float_as_uint(__fmul_rn(16.0f, __fmul_rn(h, h))) - ((uint32_t)(kTileBins - 1) << 20);
+        const float top = 16.0f * 9.0f / 3.14159265f * (float)(a.k + 1) * h * h / (float)max(seq.total, 1);
+        U.first = (__float_as_uint(fminf(top, 4.0f * h * h)) >> kTileShift) - (uint32_t)(kTileBins - 1);
     }
 }
 
 // Persistent: each half-warp claims batches (up to 16 queries of one unit)
 // one at a time; both halves run their batches together.
-template <bool kBatch, int S>
-__global__ void __launch_bounds__(kTileWarps * 32, 16) k_knn_tile(KnnArgs a, TileArgs t) {
-    constexpr int kCap = tile_cap<S>();
-    constexpr size_t kWarpBytes = tile_warp_bytes<S>();
+//
+// Bound: latency with few warps (a block of ~600 candidates is streamed twice
+// from shared memory, 16 at a time), then instruction issue.  Before the kept
+// candidates became one word each and were sorted by a network, 35 % of the
+// time went to fetching their distances again and to insertion sorts whose
+// steps differ from lane to lane, 29 % to the bucket places of pass 2.  One
+// B200, kNN stage: 4M superquadrics, k = 40: 12.18 -> 8.37 ms; 4M sheets, k =
+// 64: 16.73 -> 9.28; 1M superquadrics, k = 20: 2.55 -> 1.92.
+template <bool kBatch, typename Form>
+__global__ void __launch_bounds__(kTileWarps * 32, Form::kWarps) k_knn_tile(KnnArgs a, TileArgs t) {
+    constexpr int S = Form::S, kKeep = Form::kKeep;
+    constexpr size_t kWarpBytes = tile_warp_bytes<Form>();
+    constexpr uint32_t kPosMask = (1u << kTilePosBits) - 1u;
     extern __shared__ __align__(16) unsigned char s_tile[];
     grid_dependency_wait();
     grid_dependents_launch();
@@ -532,9 +641,9 @@ __global__ void __launch_bounds__(kTileWarps * 32, 16) k_knn_tile(KnnArgs a, Til
     const int hl = lane & 15, hf = lane >> 4;
     unsigned char* base = s_tile + (size_t)w * kWarpBytes;
     uint32_t* hist = reinterpret_cast<uint32_t*>(base);
-    uint16_t* bpos = reinterpret_cast<uint16_t*>(base + (size_t)tile_rows<S>() * 32 * 4);
-    float4* chunk = reinterpret_cast<float4*>(bpos + (size_t)kCap * 32) + 16 * hf;
-    int* s_pref = reinterpret_cast<int*>(reinterpret_cast<float4*>(bpos + (size_t)kCap * 32) + 32) + 32 * hf;
+    float* stages = reinterpret_cast<float*>(base + (size_t)tile_rows<Form>() * 32 * 4);
+    float* stage = stages + kTileStage * hf;
+    int* s_pref = reinterpret_cast<int*>(stages + 2 * kTileStage) + 32 * hf;
     int* s_start = s_pref + 16;
     uint32_t* hcol = hist + lane;
     unsigned long long evals = 0;
@@ -542,10 +651,10 @@ __global__ void __launch_bounds__(kTileWarps * 32, 16) k_knn_tile(KnnArgs a, Til
     // First the ring search (k_knn_plain's code, one query per warp) of the
     // queries no level selected, while the other warps already search
     // batches, so that the long ones do not end the search.  Its scratch lies
-    // in the kept-candidate space.  (Queries that fail the checks run it in a
+    // in the bucket space.  (Queries that fail the checks run it in a
     // separate launch at the ring kernel's own occupancy: measured faster than
     // running them here, between batches.)
-    int* r_pref = reinterpret_cast<int*>(bpos);
+    int* r_pref = reinterpret_cast<int*>(hist);
     int* r_start = r_pref + 32;
     float* r_md = reinterpret_cast<float*>(r_start + 32);
     int* r_mp = reinterpret_cast<int*>(r_md + 32 * S);
@@ -585,7 +694,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 16) k_knn_tile(KnnArgs a, Til
     U.seq.m = 0;
     U.seq.total = 0;
     U.order = nullptr;
-    U.lo = 0u;
+    U.first = 0u;
     U.l = -1;
 #pragma unroll
     for (int t = 0; t < 9; t++) {
@@ -617,7 +726,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, 16) k_knn_tile(KnnArgs a, Til
         const float4 pq = act ? p4[q] : make_float4(3e18f, 3e18f, 3e18f, 0.f);
         const int total = take ? U.seq.total : 0;
         const int steps = (max(total, __shfl_xor_sync(0xffffffffu, total, 16)) + 15) >> 4;
-        const uint32_t lo = U.lo;
+        const uint32_t first = U.first;
+        const uint32_t bins = (uint32_t)__cvta_generic_to_shared(hcol) - (first << 7);  // tile_addr's base
         // The smallest bucket of each group of g steps over the half's lanes
         // (one byte per group in the half's scratch, which the unit set-up no
         // longer needs): pass 2 visits only the groups that can hold a
@@ -631,39 +741,37 @@ __global__ void __launch_bounds__(kTileWarps * 32, 16) k_knn_tile(KnnArgs a, Til
         s_pref[hl + 16] = -1;
         __syncwarp();
         // pass 1: bucket counts (the query itself included, at distance 0)
-        tile_stream16(U, take, steps, p4, chunk, hl, hf, [&](int st) {
-            uint32_t bk[16];
+        tile_stream16(U, take, steps, p4, stage, hl, hf, [&](int st) {
+            float d[16], mnd = 3.0e38f;
+            tile_distances(stage, pq, d);
 #pragma unroll
             for (int j = 0; j < 16; j++) {
-                const float4 c = chunk[j];
-                bk[j] = tile_bin(fs_dist3(pq.x, pq.y, pq.z, c.x, c.y, c.z), lo);
+                d[j] = tile_clamp(d[j], first);
+                mnd = fminf(mnd, d[j]);
             }
 #pragma unroll
-            for (int j = 0; j < 16; j++) atomicAdd(hcol + bk[j] * 32, 1u);
-            uint32_t mn = bk[0];
-#pragma unroll
-            for (int j = 1; j < 16; j++) mn = min(mn, bk[j]);
-            mn = __reduce_min_sync(hmask, mn);
+            for (int j = 0; j < 16; j++) shared_inc(tile_addr(d[j], bins));
+            const uint32_t mn = (__reduce_min_sync(hmask, __float_as_uint(mnd)) >> kTileShift) - first;
             if (hl == 0 && st < steps_h) {
                 const int gi = st >> gs;
                 mb[gi] = (uint8_t)min((uint32_t)mb[gi], mn);
             }
         });
-        // bucket offsets and the bucket b* of the (k+1)-th distance other
-        // than the query's own
+        // the bucket b* of the (k+1)-th distance other than the query's own
         int cum = 0, bstar = -1, m = 0;
+        const int low = (int)hcol[0];  // nearer than the bucket range
 #pragma unroll 8
         for (int b = 0; b < kTileBins; b++) {
-            const int c = (int)hcol[b * 32];
-            hcol[b * 32] = (uint32_t)cum;
-            cum += c;
+            cum += (int)hcol[b * 32];
             if (bstar < 0 && cum >= k + 2) { bstar = b; m = cum; }
         }
-        bool ok = act && bstar >= 0 && bstar < kTileBins - 1 && m <= kCap;
-        const float T = ok ? __uint_as_float(lo + ((uint32_t)(bstar + 1) << 20)) : 0.0f;
-        // pass 2: the candidates of buckets <= b*, in bucket order, from the
-        // step groups whose smallest bucket is at most the half's largest b*
+        bool ok = act && bstar >= 0 && bstar < kTileBins - 1 && m <= kKeep && low <= kTileMaxUnsorted;
+        const float T = ok ? __uint_as_float((first + (uint32_t)bstar + 1u) << kTileShift) : 0.0f;
+        // pass 2: the candidates of buckets <= b* (over the spent counts), from the step
+        // groups whose smallest bucket is at most the half's largest b*
         const int bmax = __reduce_max_sync(hmask, ok ? bstar : -1);
+        const uint32_t lo = first << kTileShift;
+        uint32_t* next = hcol;
         auto nxt = [&](int st) {
             int u = st + 1;
             while (u < steps_h) {
@@ -673,61 +781,69 @@ __global__ void __launch_bounds__(kTileWarps * 32, 16) k_knn_tile(KnnArgs a, Til
             }
             return min(u, steps_h);
         };
-        tile_stream16_seq(U, nxt(-1), steps_h, nxt, p4, chunk, hl, hf, [&](int st) {
+        tile_stream16_seq(U, nxt(-1), steps_h, nxt, p4, stage, hl, hf, [&](int st) {
+            float d[16];
+            tile_distances(stage, pq, d);
 #pragma unroll
-            for (int j0 = 0; j0 < 16; j0 += 8) {
-                float dd[8];
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const float4 c = chunk[j0 + j];
-                    dd[j] = fs_dist3(pq.x, pq.y, pq.z, c.x, c.y, c.z);
-                }
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    if (dd[j] < T) {
-                        const uint32_t s = atomicAdd(hcol + tile_bin(dd[j], lo) * 32, 1u);
-                        bpos[tile_slot((int)s, lane)] = (uint16_t)(st * 16 + j0 + j);
-                    }
+            for (int j = 0; j < 16; j++) {
+                if (d[j] < T) {
+                    const uint32_t u = max(__float_as_uint(d[j]), lo) - lo;  // 26 bits
+                    *next = ((u << 6) & ~kPosMask) | (uint32_t)(st * 16 + j);
+                    next += 32;
                 }
             }
         });
+        {
+            uint32_t v[kKeep];
+#pragma unroll
+            for (int i = 0; i < kKeep; i++) v[i] = ok && i < m ? hcol[i * 32] : 0xffffffffu;
+            SortNet<kKeep>::sort(v);
+#pragma unroll
+            for (int i = 0; i < kKeep; i++) hcol[i * 32] = v[i];
+        }
+        // the point of a word, and its exact distance
+        auto point = [&](uint32_t word) { return tile_point((int)(word & kPosMask), U); };
+        auto exact = [&](uint32_t word) {
+            const float4 v = __ldg(p4 + point(word));
+            return fs_dist3(pq.x, pq.y, pq.z, v.x, v.y, v.z);
+        };
         float kth = 0.0f;
         int reached = 0;
-        int self = 0;  // slot of the query itself after sorting; entry i of the list is slot i + (i >= self)
+        int self = 0;  // the query's own word; entry i of the list is word i + (i >= self)
         if (ok) {
-            // the kept candidates' distances, into the bucket space (its offsets are spent)
-#pragma unroll 4
-            for (int i = 0; i < m; i++) {
-                const float4 v = __ldg(p4 + tile_point(bpos[tile_slot(i, lane)], U));
-                hcol[i * 32] = __float_as_uint(fs_dist3(pq.x, pq.y, pq.z, v.x, v.y, v.z));
-            }
-            // sorted by (distance, block position); only candidates of one bucket are out of order
+            // words that agree above the position, by (distance, block position)
+            uint32_t before = hcol[0];
             for (int i = 1; i < m; i++) {
-                const uint32_t ed = hcol[i * 32], ei = bpos[tile_slot(i, lane)];
-                int j = i;
-                while (j > 0) {
-                    const uint32_t gd = hcol[(j - 1) * 32], gi = bpos[tile_slot(j - 1, lane)];
-                    if (gd < ed || (gd == ed && gi < ei)) break;
-                    hcol[j * 32] = gd;
-                    bpos[tile_slot(j, lane)] = (uint16_t)gi;
-                    j--;
+                uint32_t w = hcol[i * 32];
+                if ((w ^ before) <= kPosMask) {
+                    const float d = exact(w);
+                    int j = i;
+                    while (j > 0) {
+                        const uint32_t g = hcol[(j - 1) * 32];
+                        if ((g ^ w) > kPosMask) break;
+                        const float e = exact(g);
+                        if (e < d || (e == d && g < w)) break;
+                        hcol[j * 32] = g;
+                        j--;
+                    }
+                    hcol[j * 32] = w;
+                    w = hcol[i * 32];
                 }
-                hcol[j * 32] = ed;
-                bpos[tile_slot(j, lane)] = (uint16_t)ei;
+                before = w;
             }
             // the query sits among the distance-0 entries at the front
-            while (self < m - 1 && tile_point(bpos[tile_slot(self, lane)], U) != q) self++;
+            while (self < m - 1 && point(hcol[self * 32]) != q) self++;
             // (1) the k+1 smallest distances pairwise distinct
             uint32_t prev = hcol[(self == 0 ? 1 : 0) * 32];
             for (int i = 1; i <= k && ok; i++) {
                 const uint32_t cur = hcol[(i + (i >= self)) * 32];
-                ok = cur != prev;
+                if ((cur ^ prev) <= kPosMask) ok = exact(cur) != exact(prev);
                 prev = cur;
             }
         }
         if (ok) {
             const int l = U.l;
-            kth = __uint_as_float(hcol[(k - 1 + (k - 1 >= self)) * 32]);
+            kth = exact(hcol[(k - 1 + (k - 1 >= self)) * 32]);
             const uint32_t c0 = __float_as_uint(pq.w);
             const int cq[3] = {(int)(c0 & 1023u), (int)((c0 >> 10) & 1023u), (int)((c0 >> 20) & 1023u)};
             // (2) the k-th ball inside the searched block
@@ -756,7 +872,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 16) k_knn_tile(KnnArgs a, Til
                 }
                 if (!ball_in_box(np, pq, kth, lo3, end3)) {
                     for (int i = 0; i < k && ok; i++) {
-                        const int p = tile_point(bpos[tile_slot(i + (i >= self), lane)], U);
+                        const int p = point(hcol[(i + (i >= self)) * 32]);
                         ok = visit_step(__float_as_uint(p4[p].w), c0) <= sf;
                     }
                 }
@@ -769,7 +885,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, 16) k_knn_tile(KnnArgs a, Til
         }
         if (ok) {
             int* row = A.lists + (size_t)q * k;
-            for (int i = 0; i < k; i++) row[i] = tile_point(bpos[tile_slot(i + (i >= self), lane)], U);
+#pragma unroll 4
+            for (int i = 0; i < k; i++) row[i] = point(hcol[(i + (i >= self)) * 32]);
             if (A.kth_out) A.kth_out[q] = kth;
             if (A.qlevel) A.qlevel[q] = (uint8_t)reached;
             if constexpr (kBatch) {
@@ -856,9 +973,9 @@ inline egt_status tile_prepare(egt_handle* h, TileArgs* t) {
 
 // Assignment, batching and the tile kernel (with the ring search of the
 // queries no level selected); the uncertified queries are left in t.ring2.
-template <bool kBatch, int S>
+template <bool kBatch, typename Form>
 egt_status tile_kernel_launch(const KnnArgs& a, const TileArgs& t, cudaStream_t st) {
-    constexpr size_t smem = tile_warp_bytes<S>() * kTileWarps;
+    constexpr size_t smem = tile_warp_bytes<Form>() * kTileWarps;
     static std::mutex mu;
     static std::map<int, unsigned> waves;  // per device: blocks of one resident wave
     int dev = 0;
@@ -870,17 +987,17 @@ egt_status tile_kernel_launch(const KnnArgs& a, const TileArgs& t, cudaStream_t 
         if (it != waves.end()) G = it->second;
     }
     if (!G) {
-        EGT_CUDA_TRY(cudaFuncSetAttribute(k_knn_tile<kBatch, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        EGT_CUDA_TRY(cudaFuncSetAttribute(k_knn_tile<kBatch, Form>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
         int sms = 0, per = 0;
         EGT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        EGT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_knn_tile<kBatch, S>, kTileWarps * 32,
+        EGT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_knn_tile<kBatch, Form>, kTileWarps * 32,
                                                                     smem));
         G = (unsigned)std::max(1, sms * std::max(per, 1));
         std::lock_guard<std::mutex> lock(mu);
         waves[dev] = G;
     }
-    return launch_dependent(k_knn_tile<kBatch, S>, dim3(G), dim3(kTileWarps * 32), smem, st, a, t);
+    return launch_dependent(k_knn_tile<kBatch, Form>, dim3(G), dim3(kTileWarps * 32), smem, st, a, t);
 }
 
 // kmax: the largest k among the queries the tile search takes.
@@ -892,7 +1009,9 @@ egt_status tile_launch(const KnnArgs& a, const TileArgs& t, int kmax, cudaStream
     const unsigned Gu = (unsigned)std::min<int64_t>(4096, (npts + T - 1) / T);
     EGT_TRY(launch_dependent(k_tile_count<kBatch>, dim3(Gu), dim3(T), 0, st, a, t));
     EGT_TRY(launch_dependent(k_tile_gather<kBatch>, dim3(Gu), dim3(T), 0, st, a, t));
-    return kmax <= kTileMaxK2 ? tile_kernel_launch<kBatch, 2>(a, t, st) : tile_kernel_launch<kBatch, 3>(a, t, st);
+    if (kmax <= TileForm1::kMaxK) return tile_kernel_launch<kBatch, TileForm1>(a, t, st);
+    if (kmax <= TileForm2::kMaxK) return tile_kernel_launch<kBatch, TileForm2>(a, t, st);
+    return tile_kernel_launch<kBatch, TileForm3>(a, t, st);
 }
 
 }  // namespace
