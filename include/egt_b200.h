@@ -164,10 +164,10 @@ egt_status egt_get_knn_host(egt_handle* h, int* knn_host, void* stream);
  * overlapped: the queries are searched in chunks of original rows, and each
  * chunk's rows are copied to knn_host (n*k ints; pinned memory lets the copy
  * overlap) while the next chunk is searched.  The handle's lists are those
- * of egt_knn.  The chunks run the ring search in every mode but
- * EGT_KNN_LEARNED, where the search and the copy run one after the other
- * (the cell-tile search finishes cell by cell, not in row order, so its copy
- * could not start early). */
+ * of egt_knn.  Where egt_knn takes the cell-tile search, and in
+ * EGT_KNN_LEARNED, the search and the copy run one after the other (the
+ * cell-tile search finishes cell by cell, not in row order, so its copy could
+ * not start early). */
 egt_status egt_knn_host(egt_handle* h, int k, int* knn_host, void* stream);
 
 /* Query-vs-reference kNN against the handle's points:

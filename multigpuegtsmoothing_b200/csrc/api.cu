@@ -259,11 +259,12 @@ egt_status egt_knn_host(egt_handle* h, int k, int* knn_host, void* stream) {
     EGT_CUDA_TRY(cudaSetDevice(h->cfg.device));
     bind_stream(h, stream);
     // The chunked ring search overlaps each chunk's copy with the next chunk's
-    // search.  The cell-tile search completes cell by cell, not in row order,
-    // so its copy could only follow the whole search: measured slower end to
-    // end (4M points, k = 40: 33.6 ms against 27.2 ms), so EGT_KNN_TILE uses
-    // the chunked ring search here.
-    if (h->cfg.knn_mode == EGT_KNN_LEARNED) {  // no chunked form: search, then copy
+    // search.  The cell-tile search completes cell by cell, not in row order, so
+    // its copy can only follow the whole search, and still ends sooner wherever
+    // egt_knn takes it (from pinned points to pinned lists, chunked ring against
+    // tiles then copy: 60K points, k = 40 1.00 -> 0.81 ms; 1M, k = 10 3.76 ->
+    // 3.24, k = 40 6.85 -> 5.94, k = 64 13.8 -> 9.2; 4M, k = 40 25.5 -> 22.8).
+    if (h->cfg.knn_mode == EGT_KNN_LEARNED || (h->cfg.knn_mode == EGT_KNN_TILE && knn_tiles(h->n, k))) {
         EGT_TRY(egt_knn(h, k, stream));
         return egt_get_knn_host(h, knn_host, stream);
     }

@@ -277,6 +277,7 @@ inline egt_status reset_knn_counters(egt_handle* h) {
 }
 egt_status set_threshold(egt_handle* h, float thres);
 egt_status run_knn(egt_handle* h, int k);
+bool knn_tiles(int64_t n, int k);
 egt_status run_knn_host(egt_handle* h, int k, int* host);
 egt_status run_knn_query(egt_handle* h, const float* q_host, int64_t nq, int k, int* out_host, int64_t* invalid);
 egt_status run_knn_learned(egt_handle* h, int k, const egt_proposal* p);

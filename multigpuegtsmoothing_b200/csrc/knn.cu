@@ -860,6 +860,9 @@ static egt_status tile_search(egt_handle* h, const KnnArgs& a, cudaStream_t st) 
     return knn_launch(ar, st);
 }
 
+// Whether EGT_KNN_TILE takes the cell-tile search.
+bool knn_tiles(int64_t n, int k) { return tile_takes(n, k); }
+
 egt_status run_knn(egt_handle* h, int k) {
     cudaStream_t st = h->stream;
     KnnArgs a;
