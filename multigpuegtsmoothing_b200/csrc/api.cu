@@ -222,9 +222,10 @@ egt_status egt_update_points_device(egt_handle* h, const float* xyz_dev, void* s
     h->have_csr = false;
     if (h->nrm) { dev_free(h, h->nrm); h->nrm = nullptr; }
     EGT_TRY(build_grid(h, xyz_dev, kMaxLevels));
-    // the caller may reuse xyz_dev on any stream: it has been read
-    EGT_CUDA_TRY(cudaEventSynchronize(h->ev[kEvRead]));
-    return EGT_OK;
+    // The whole build is waited for, not the reading of xyz_dev alone: the next
+    // call may name another stream, and a holder of the views' pointers may read
+    // them on any stream.
+    return fetch_norm(h);
 }
 
 int64_t egt_kernel_launches(void) { return g_launches; }
@@ -494,10 +495,6 @@ egt_status egt_free_device(void* p) {
 egt_status egt_get_views(egt_handle* h, egt_views* v) {
     EGT_TRY(check_handle(h));
     if (!v) { set_error("egt_get_views: null output"); return EGT_ERR_ARG; }
-    if (!h->norm_valid && h->d_norm) {
-        EGT_CUDA_TRY(cudaSetDevice(h->cfg.device));
-        EGT_TRY(fetch_norm(h));
-    }
     v->x = h->x;
     v->y = h->y;
     v->z = h->z;

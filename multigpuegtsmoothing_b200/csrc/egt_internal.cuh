@@ -169,8 +169,6 @@ struct LevelDev {
     int2* row_range = nullptr; // [B*B] [first, last) cell of each (y,z) row
 };
 
-constexpr int kEvRead = 16;  // egt_handle::ev
-
 struct Scratch {
     void* ptr = nullptr;
     size_t bytes = 0;
@@ -194,7 +192,6 @@ struct egt_handle {
     int* perm = nullptr;         // [n] sorted -> original
     egt::NormParams* d_norm = nullptr;
     egt::NormParams norm{};      // host copy (fetch_norm)
-    bool norm_valid = false;
     egt::LevelDev lv[egt::kMaxLevels];  // slices of grid_mem
     void* grid_mem = nullptr;    // row ranges of all levels, then their cells and orders
     size_t row_bytes = 0;        // bytes of the row ranges
@@ -252,7 +249,7 @@ struct egt_handle {
     const uint16_t* cloud_of = nullptr;
     int cloud_bits = 0;
     // timing
-    cudaEvent_t ev[17] = {};     // stage timing pairs; kEvRead: the grid build has read its input
+    cudaEvent_t ev[16] = {};     // stage timing pairs
     egt_timings tm{};
     egt::Scratch scratch;
 };

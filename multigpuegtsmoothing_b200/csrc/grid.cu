@@ -427,12 +427,11 @@ egt_status scratch_reserve(egt_handle* h, size_t bytes, void** out) {
 }
 
 // Full grid build from device AoS xyz (n points).  levels = number of
-// hierarchy levels to build (8 for point clouds, 1 for meshes).  xyz is read
-// until h->ev[kEvRead].
+// hierarchy levels to build (8 for point clouds, 1 for meshes).  Enqueued
+// only: fetch_norm waits for it.
 egt_status build_grid(egt_handle* h, const float* xyz, int levels) {
     const int64_t n = h->n;
     cudaStream_t st = h->stream;
-    h->norm_valid = false;
     EGT_TRY(level_memory(h, levels));
     h->levels_built = levels;
     const int64_t tiles = radix_tiles(n), ttiles = (n + kTableTile - 1) / kTableTile;
@@ -495,7 +494,6 @@ egt_status build_grid(egt_handle* h, const float* xyz, int levels) {
     }
     EGT_TRY(launch_dependent(k_gather_sorted, dim3(gk), dim3(kT), 0, st, xyz, h->perm, U(o_key0), n, h->p4, h->x, h->y,
                              h->z, h->cell0, h->d_norm, levels > 1 ? U(o_hist) : nullptr));
-    EGT_CUDA_TRY(cudaEventRecord(h->ev[kEvRead], st));
     TableBatch tb{};
     tb.n = (int)n;
     tb.polls = kRadixPolls;
@@ -539,12 +537,10 @@ egt_status build_grid(egt_handle* h, const float* xyz, int levels) {
     return EGT_OK;
 }
 
-// The host's copy of the normalisation cube.
+// The host's copy of the normalisation cube; waits for the grid build.
 egt_status fetch_norm(egt_handle* h) {
-    if (h->norm_valid) return EGT_OK;
     EGT_CUDA_TRY(cudaMemcpyAsync(&h->norm, h->d_norm, sizeof(NormParams), cudaMemcpyDeviceToHost, h->stream));
     EGT_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    h->norm_valid = true;
     return EGT_OK;
 }
 
