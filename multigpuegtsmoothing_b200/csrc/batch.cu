@@ -1143,12 +1143,6 @@ egt_status egt_batch_get_timings(egt_batch* b, egt_batch_timings* t) {
     EGT_CUDA_TRY(cudaStreamSynchronize(h->stream));
     std::vector<unsigned long long> ctr((size_t)kCtrWords * b->count);
     EGT_CUDA_TRY(cudaMemcpy(ctr.data(), b->d_ctr, sizeof(unsigned long long) * ctr.size(), cudaMemcpyDeviceToHost));
-    unsigned long long fail = 0;
-    EGT_CUDA_TRY(cudaMemcpy(&fail, h->d_counters + kCtrTaubinFail, sizeof(fail), cudaMemcpyDeviceToHost));
-    if (fail) {
-        set_error("egt_batch: a wait of the smoothing loop expired; the positions are NaN");
-        return EGT_ERR_TIMEOUT;
-    }
     b->tm.knn_ms = elapsed_ms(h->ev[2], h->ev[3]);
     b->tm.egt_ms = elapsed_ms(h->ev[4], h->ev[5]);
     b->tm.taubin_ms = elapsed_ms(h->ev[6], h->ev[7]);

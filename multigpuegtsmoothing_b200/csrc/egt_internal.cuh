@@ -135,11 +135,12 @@ constexpr int kCtrNcells = 0;     // [0..7]  occupied cells per level (int in a 
 constexpr int kCtrExtents = 16;   // [16..18] six packed u32 min/max words
 constexpr int kCtrEgtTests = 24;    // EGT filter: ellipsoid tests of the last filter run
 constexpr int kCtrSpillTiles = 25;  // Taubin tiles that gather from global memory (too large to stage)
-constexpr int kCtrTaubinFail = 26;  // a wait of the resident Taubin loop expired
+constexpr int kCtrTaubinFail = 26;  // a wait of the resident Taubin loop expired (until it is redone)
 constexpr int kCtrFlag = 27;      // generic loop flag
 constexpr int kCtrNormFallback = 28;  // normals re-solved in FP64
 constexpr int kCtrMsf = 29;       // spanning-forest edges
 constexpr int kCtrComps = 30;     // orientation components
+constexpr int kCtrTaubinRedo = 31;  // resident Taubin loops that gave up and were redone
 constexpr int kCtrMaxPop = 32;    // [32..39] largest cell population per level (grid build)
 // counters of the last kNN, reset together
 constexpr int kCtrKnn = 40, kCtrKnnWords = 14;
@@ -235,6 +236,7 @@ struct egt_handle {
     int* t_soff = nullptr;       // [tiles * 9] slice offsets into t_loc, then the table size
     uint32_t* t_adj = nullptr;   // small clouds: bits of the tiles each tile shares edges with (k_taubin_resident)
     uint32_t taubin_tag = 0;     // tag of the next resident loop's first half-step
+    int resident_polls = 0;      // polls of one wait of the resident loop (0: kResidentPolls)
     int64_t t_tiles = 0;         // tiles the tables above are sized for
     uint64_t csr_version = 0;    // bumped whenever the CSR is rebuilt
     uint64_t m_version = ~0ull;  // CSR version the Morton copy was built from

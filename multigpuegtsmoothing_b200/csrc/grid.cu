@@ -139,7 +139,6 @@ __global__ void __launch_bounds__(kT) k_extents(const float* __restrict__ xyz, i
         *out = finalize_norm(acc, eps, thres0, n);
     }
     if (threadIdx.x < kMaxLevels) counters[kCtrMaxPop + threadIdx.x] = 0ull;  // k_tables fills them
-    if (threadIdx.x == 0) counters[kCtrTaubinFail] = 0ull;  // these are new positions
 }
 
 // GRIDCUDAKNNSELF_COMPACT's threshold scaling (GridKNNCuda.cu:2324-2325):

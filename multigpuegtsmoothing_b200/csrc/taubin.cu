@@ -301,10 +301,10 @@ __device__ __forceinline__ float4 load_tagged(const float4* p) {
 // of which it reads one row's tag.
 //
 // The blocks wait on one another, so the grid is launched cooperatively, one
-// block per tile, all resident.  A wait that does not end (kResidentPolls)
-// sets *fail and every block leaves; k_scatter_morton then writes NaN
-// positions, and the calls that read the handle's counters return
-// EGT_ERR_TIMEOUT.
+// block per tile, all resident.  A wait that does not end (max_polls) sets
+// *fail and every block leaves; k_taubin_redo then computes the same half-steps
+// from the positions the loop began with, so a call never ends with anything
+// else than its result.
 //
 // Bound: the latency of a half-step (store to L2, load from L2, the rows'
 // serial sums).  36K points 2.2 us per half-step, 131K-vertex mesh 2.1, 2,500
@@ -321,12 +321,13 @@ __global__ void __launch_bounds__(kTile, 4) k_taubin_resident(
     float4* buf_a, float4* buf_b, const int* __restrict__ off, const int* __restrict__ col,
     const int* __restrict__ t_uni, const uint32_t* __restrict__ t_loc, const int* __restrict__ t_nu,
     const int* __restrict__ t_soff, const uint32_t* __restrict__ t_adj, int adj_words, int n, int steps, float lambda,
-    float mu, uint32_t tag0, unsigned long long* __restrict__ fail) {
+    float mu, uint32_t tag0, int max_polls, unsigned long long* __restrict__ fail) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint16_t s_dep[kResidentMaxTiles];
     __shared__ uint32_t s_read[kResidentMaxTiles / 32];  // tiles this one reads from
     __shared__ int16_t s_own[kTile];                     // staged slot of each of the tile's own rows (-1: none)
     __shared__ int s_ndep;
+    if (*(volatile unsigned long long*)fail) return;  // an earlier part of the loop gave up
     const int tile = blockIdx.x, lane = threadIdx.x & 31;
     float4* const s_pos = reinterpret_cast<float4*>(smem);  // two stages
     uint32_t* const s_loc = reinterpret_cast<uint32_t*>(smem + 2 * kUCap * sizeof(float4));
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(kTile, 4) k_taubin_resident(
     auto wait_for = [&](const float4* q, uint32_t tag) {
         float4 v = load_tagged(q);
         while (__float_as_uint(v.w) != tag && !lost) {
-            if (++polls >= kResidentPolls || ((polls & 1023) == 0 && *(volatile unsigned long long*)fail)) lost = true;
+            if (++polls >= max_polls || ((polls & 1023) == 0 && *(volatile unsigned long long*)fail)) lost = true;
             v = load_tagged(q);
         }
         return v;
@@ -418,6 +419,43 @@ __global__ void __launch_bounds__(kTile, 4) k_taubin_resident(
             store_tagged(pout + i, p);
             if (own >= 0) s_pos[((step & 1) ^ 1) * kUCap + own] = p;
         }
+    }
+}
+
+// The half-steps of a resident loop that gave up (*fail; otherwise nothing),
+// from the positions p4 it began with: one block, which waits for no other, the
+// general half-step's sums in its order, so the same positions bit for bit.  Clears
+// *fail and counts the call in *redone.
+constexpr int kRedoThreads = 1024;
+__global__ void __launch_bounds__(kRedoThreads, 1) k_taubin_redo(const float4* __restrict__ p4,
+                                                                 const int* __restrict__ perm, float4* buf_a,
+                                                                 float4* buf_b, const int* __restrict__ off,
+                                                                 const int* __restrict__ col, int n, int64_t steps,
+                                                                 float lambda, float mu, unsigned long long* fail,
+                                                                 unsigned long long* redone) {
+    grid_dependency_wait();
+    if (!*(volatile unsigned long long*)fail) return;
+    for (int i = threadIdx.x; i < n; i += kRedoThreads) {
+        float4 v = p4[perm[i]];
+        v.w = __uint_as_float(kNoTag);
+        buf_a[i] = v;
+        buf_b[i] = v;
+    }
+    __syncthreads();
+    for (int64_t step = 0; step < steps; step++) {
+        const float4* pin = (step & 1) ? buf_b : buf_a;
+        float4* pout = (step & 1) ? buf_a : buf_b;
+        for (int i = threadIdx.x; i < n; i += kRedoThreads) {
+            const float4 p = pin[i];
+            float cx = 0.0f, cy = 0.0f, cz = 0.0f, sum = 0.0f;
+            for (int e = off[i]; e < off[i + 1]; e++) accumulate(p.x, p.y, p.z, pin[col[e]], cx, cy, cz, sum);
+            pout[i] = finish(p, cx, cy, cz, sum, (step & 1) ? mu : lambda);
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        *fail = 0ull;
+        *redone += 1ull;
     }
 }
 
@@ -630,15 +668,13 @@ __global__ void k_gather_morton(const float4* __restrict__ p4, const int* __rest
     mp[i] = v;
 }
 
-// failed: a resident loop gave up (k_taubin_resident); its positions are no result.
 __global__ void k_scatter_morton(const float4* __restrict__ mp, const int* __restrict__ perm, int n,
                                  float4* __restrict__ p4, float* __restrict__ x, float* __restrict__ y,
-                                 float* __restrict__ z, const uint32_t* __restrict__ cell0,
-                                 const unsigned long long* __restrict__ failed) {
+                                 float* __restrict__ z, const uint32_t* __restrict__ cell0) {
+    grid_dependency_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float4 v = mp[i];
-    if (*failed) v.x = v.y = v.z = __int_as_float(0x7fffffff);
     const int s = perm[i];
     v.w = __uint_as_float(cell0[s]);  // as the grid build stores it
     p4[s] = v;
@@ -792,11 +828,15 @@ static egt_status morton_prepare(egt_handle* h) {
     return EGT_OK;
 }
 
-// The whole loop over a cloud whose tiles are all resident at once.
-static egt_status resident_loop(egt_handle* h, int iters, float lambda, float mu, cudaStream_t st) {
+// The whole loop over a cloud whose tiles are all resident at once.  *left: the
+// iterations still to do (iters: the launch was refused, as where a context has
+// fewer SMs than the device).
+static egt_status resident_loop(egt_handle* h, int iters, float lambda, float mu, cudaStream_t st, int* left) {
     const int n = (int)h->n, tiles = (n + kTile - 1) / kTile;
-    for (int left = iters; left > 0;) {  // long loops in several launches: the tags stay far from wrapping
-        const int part = std::min(left, 1 << 24);
+    const int max_polls = h->resident_polls > 0 ? h->resident_polls : kResidentPolls;
+    *left = iters;
+    while (*left > 0) {  // long loops in several launches: the tags stay far from wrapping
+        const int part = std::min(*left, 1 << 24);
         if (h->taubin_tag > 0xf0000000u) {  // (kNoTag and tags of long ago are never waited for)
             h->taubin_tag = 0;
             EGT_CUDA_TRY(cudaMemsetAsync(h->m_pb, 0xff, sizeof(float4) * (size_t)n, st));
@@ -811,16 +851,29 @@ static egt_status resident_loop(egt_handle* h, int iters, float lambda, float mu
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        EGT_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_taubin_resident, h->m_p, h->m_pb, (const int*)h->m_off,
-                                        (const int*)h->m_col, (const int*)h->t_uni, (const uint32_t*)h->t_loc,
-                                        (const int*)h->t_nu, (const int*)h->t_soff, (const uint32_t*)h->t_adj,
-                                        adj_words(tiles), n, 2 * part, lambda, mu, h->taubin_tag,
-                                        h->d_counters + kCtrTaubinFail));
+        const cudaError_t e = cudaLaunchKernelEx(
+            &cfg, k_taubin_resident, h->m_p, h->m_pb, (const int*)h->m_off, (const int*)h->m_col,
+            (const int*)h->t_uni, (const uint32_t*)h->t_loc, (const int*)h->t_nu, (const int*)h->t_soff,
+            (const uint32_t*)h->t_adj, adj_words(tiles), n, 2 * part, lambda, mu, h->taubin_tag, max_polls,
+            h->d_counters + kCtrTaubinFail);
+        if (*left == iters && (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported)) {
+            cudaGetLastError();
+            return EGT_OK;
+        }
+        EGT_CUDA_TRY(e);
         EGT_LAUNCH_CHECK();
         h->taubin_tag += 2u * (uint32_t)part;
-        left -= part;
+        *left -= part;
     }
-    return EGT_OK;
+    return launch_dependent(k_taubin_redo, dim3(1), dim3(kRedoThreads), 0, st, h->p4, h->m_perm, h->m_p, h->m_pb,
+                            h->m_off, h->m_col, n, 2 * (int64_t)iters, lambda, mu, h->d_counters + kCtrTaubinFail,
+                            h->d_counters + kCtrTaubinRedo);
+}
+
+static egt_status scatter_launch(egt_handle* h, cudaStream_t st) {
+    const int n = (int)h->n;
+    return launch_dependent(k_scatter_morton, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, h->m_p, h->m_perm,
+                            n, h->p4, h->x, h->y, h->z, h->cell0);
 }
 
 egt_status run_taubin(egt_handle* h, int iters, float lambda, float mu) {
@@ -860,12 +913,13 @@ egt_status run_taubin(egt_handle* h, int iters, float lambda, float mu) {
         const unsigned blocks = wave[dev & 63].load();
         const int tiles = (n + kTile - 1) / kTile;
         if (h->taubin_mode == 0 && h->t_adj && tiles <= (int)resident[dev & 63].load()) {
-            EGT_TRY(resident_loop(h, iters, lambda, mu, st));
-            k_scatter_morton<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(h->m_p, h->m_perm, n, h->p4, h->x, h->y,
-                                                                           h->z, h->cell0, h->d_counters + kCtrTaubinFail);
-            EGT_LAUNCH_CHECK();
-            EGT_CUDA_TRY(cudaEventRecord(h->ev[7], st));
-            return EGT_OK;
+            int left = 0;
+            EGT_TRY(resident_loop(h, iters, lambda, mu, st, &left));
+            if (left == 0) {
+                EGT_TRY(scatter_launch(h, st));
+                EGT_CUDA_TRY(cudaEventRecord(h->ev[7], st));
+                return EGT_OK;
+            }
         }
         // every buffer the captured launches name
         const void* key[8] = {h->m_p, h->m_pb, h->t_uni, h->t_loc, h->t_nu, h->t_soff, h->m_off, h->m_col};
@@ -917,9 +971,7 @@ egt_status run_taubin(egt_handle* h, int iters, float lambda, float mu) {
             for (int i = 0; i < 2 * iters; i++) count_launch();
         }
         EGT_CUDA_TRY(cudaGraphLaunch(h->taubin_exec, st));
-        k_scatter_morton<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(h->m_p, h->m_perm, n, h->p4, h->x, h->y,
-                                                                       h->z, h->cell0, h->d_counters + kCtrTaubinFail);
-        EGT_LAUNCH_CHECK();
+        EGT_TRY(scatter_launch(h, st));
     } else {
         k_split_soa<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(h->p4, n, h->x, h->y, h->z);
         EGT_LAUNCH_CHECK();
