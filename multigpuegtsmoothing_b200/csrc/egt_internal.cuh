@@ -237,6 +237,7 @@ struct egt_handle {
     uint32_t* t_adj = nullptr;   // small clouds: bits of the tiles each tile shares edges with (k_taubin_resident)
     uint32_t taubin_tag = 0;     // tag of the next resident loop's first half-step
     int resident_polls = 0;      // polls of one wait of the resident loop (0: kResidentPolls)
+    int64_t t_spilled = -1;      // tiles of the current tables that are not staged (-1: not fetched)
     int64_t t_tiles = 0;         // tiles the tables above are sized for
     uint64_t csr_version = 0;    // bumped whenever the CSR is rebuilt
     uint64_t m_version = ~0ull;  // CSR version the Morton copy was built from

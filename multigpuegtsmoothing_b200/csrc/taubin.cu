@@ -21,8 +21,8 @@
 // Relabelling changes neither a row's neighbour order nor any value, so the
 // result is the same bit for bit.  Each half-step is a programmatic dependent
 // launch: its prologue (CSR tables only) overlaps the previous half-step.
-// Clouds whose tiles are all resident at once (592 tiles, 151K points) run the
-// loop in one launch instead (k_taubin_resident).
+// Clouds whose tiles are all resident at once (592 tiles, 151K points) and all
+// staged run the loop in one launch instead (k_taubin_resident).
 #include <algorithm>
 #include <atomic>
 #include <climits>
@@ -306,6 +306,12 @@ __device__ __forceinline__ float4 load_tagged(const float4* p) {
 // from the positions the loop began with, so a call never ends with anything
 // else than its result.
 //
+// Only for clouds whose tiles are all staged.  Rows that gather from the buffer
+// would have to poll every neighbour through L2, where the launch-per-half-step
+// loop's gathers hit L1: 50 iterations on 36K points, unfiltered lists of 40,
+// 2.06 ms so against 0.98 with launches; 100K points in clusters, 32 of 391 tiles
+// not staged, 1.60 against 0.97.
+//
 // Bound: the latency of a half-step (store to L2, load from L2, the rows'
 // serial sums).  36K points 2.2 us per half-step, 131K-vertex mesh 2.1, 2,500
 // points 1.7.  A launch per half-step: 4.1, 5.3 and 3.5 us, and 1.1 ms of host
@@ -314,14 +320,15 @@ __device__ __forceinline__ float4 load_tagged(const float4* p) {
 // cache lines).
 constexpr int kResidentPolls = 1 << 22;
 constexpr int kResidentMaxTiles = 1024;  // entries of a block's list of reading tiles
+constexpr int64_t kSmallCols = 1 << 24;  // entries (64 MB)
 constexpr uint32_t kNoTag = 0xffffffffu;  // w of positions that no resident loop wrote
 constexpr size_t kResidentSmem = 2 * kUCap * sizeof(float4) + kSellWords * sizeof(uint32_t);
 
 __global__ void __launch_bounds__(kTile, 4) k_taubin_resident(
-    float4* buf_a, float4* buf_b, const int* __restrict__ off, const int* __restrict__ col,
-    const int* __restrict__ t_uni, const uint32_t* __restrict__ t_loc, const int* __restrict__ t_nu,
-    const int* __restrict__ t_soff, const uint32_t* __restrict__ t_adj, int adj_words, int n, int steps, float lambda,
-    float mu, uint32_t tag0, int max_polls, unsigned long long* __restrict__ fail) {
+    float4* buf_a, float4* buf_b, const int* __restrict__ off, const int* __restrict__ t_uni,
+    const uint32_t* __restrict__ t_loc, const int* __restrict__ t_nu, const int* __restrict__ t_soff,
+    const uint32_t* __restrict__ t_adj, int adj_words, int n, int steps, float lambda, float mu, uint32_t tag0,
+    int max_polls, unsigned long long* __restrict__ fail) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint16_t s_dep[kResidentMaxTiles];
     __shared__ uint32_t s_read[kResidentMaxTiles / 32];  // tiles this one reads from
@@ -345,9 +352,8 @@ __global__ void __launch_bounds__(kTile, 4) k_taubin_resident(
             else atomicOr(&s_read[from >> 5], 1u << (from & 31));
         }
     }
-    if (r.nu >= 0)
-        for (int v = threadIdx.x; v < (r.ssize + 3) >> 2; v += kTile)
-            cp_async16(s_loc + 4 * v, t_loc + (size_t)tile * kSellWords + 4 * v);
+    for (int v = threadIdx.x; v < (r.ssize + 3) >> 2; v += kTile)
+        cp_async16(s_loc + 4 * v, t_loc + (size_t)tile * kSellWords + 4 * v);
     cp_async_commit();
     __syncthreads();
     for (int u = threadIdx.x; u < (int)gridDim.x; u += kTile)
@@ -402,18 +408,12 @@ __global__ void __launch_bounds__(kTile, 4) k_taubin_resident(
             }
             for (int d = threadIdx.x; d < ndep; d += kTile) wait_for(pin + s_dep[d] * kTile, tag);
         }
-        if (r.nu < 0 && i < n) {  // tile too large to stage: its rows read their neighbours from the buffer
-            for (int e = r.e0; e < r.e1; e++) {
-                const float4* q = pin + __ldg(col + e);
-                accumulate(p.x, p.y, p.z, step ? wait_for(q, tag) : *q, cx, cy, cz, sum);
-            }
-        }
         if (__syncthreads_or(lost)) {
             if (threadIdx.x == 0) atomicExch(fail, 1ull);
             break;
         }
         if (i < n) {
-            if (r.nu >= 0) tile_row(stage, ls0, len, p, cx, cy, cz, sum);
+            tile_row(stage, ls0, len, p, cx, cy, cz, sum);
             p = finish(p, cx, cy, cz, sum, (step & 1) ? mu : lambda);
             p.w = __uint_as_float(step + 1 < steps ? tag + 1u : kNoTag);
             store_tagged(pout + i, p);
@@ -491,15 +491,13 @@ __global__ void __launch_bounds__(kBuildThreads) k_tile_build(const int* __restr
     __shared__ int s_soff[kSoffWords];
     __shared__ int s_nu;
     const int tile = blockIdx.x;
-    // tile u shares an edge with this one (t_adj: symmetric bits, for k_taubin_resident)
+    // tile u shares an edge with this one (t_adj: symmetric bits, for k_taubin_resident; complete when no tile spills)
     auto joined = [&](int u) {
         atomicOr(&t_adj[(size_t)tile * adj_words + (u >> 5)], 1u << (u & 31));
         atomicOr(&t_adj[(size_t)u * adj_words + (tile >> 5)], 1u << (tile & 31));
     };
-    auto spill = [&]() {  // not staged: its neighbours are not listed, so it counts as joined to every tile
+    auto spill = [&]() {
         if (threadIdx.x == 0) { t_nu[tile] = -1; atomicAdd(spilled, 1ull); }
-        if (t_adj)
-            for (int u = threadIdx.x; u < (int)gridDim.x; u += kBuildThreads) joined(u);
     };
     const int base = tile * kTile;
     const int last = min(base + kTile, n);
@@ -739,8 +737,11 @@ static egt_status morton_prepare(egt_handle* h) {
         EGT_CUDA_TRY(dev_alloc(h, &h->m_off, sizeof(int) * (n + 1)));
     }
     if (h->m_version != h->csr_version) {
-        int64_t nnz = 0;
-        EGT_TRY(csr_nnz(h, &nnz));  // one host round trip per CSR, at set-up
+        // One host round trip per CSR, at set-up: its size, or for a small cloud,
+        // where that buffer may be as large as the lists, the spilled tiles
+        // (spilled_tiles) instead.
+        int64_t nnz = h->csr_cap;
+        if (n > kResidentMaxTiles * kTile || nnz > kSmallCols) EGT_TRY(csr_nnz(h, &nnz));
         if (h->m_cap < nnz || !h->m_col) {
             if (h->m_col) dev_free(h, h->m_col);
             h->m_col = nullptr;
@@ -817,6 +818,7 @@ static egt_status morton_prepare(egt_handle* h) {
                                                                  h->d_counters + kCtrSpillTiles);
         EGT_LAUNCH_CHECK();
         h->tm.taubin_tiles = tiles;
+        h->t_spilled = -1;
         cudaFreeAsync(kin, st);
         cudaFreeAsync(kout, st);
         cudaFreeAsync(idx, st);
@@ -825,6 +827,18 @@ static egt_status morton_prepare(egt_handle* h) {
     }
     k_gather_morton<<<G, 256, 0, st>>>(h->p4, h->m_perm, n, h->m_p);
     EGT_LAUNCH_CHECK();
+    return EGT_OK;
+}
+
+// Tiles of the current CSR that are not staged; fetched once per CSR.
+static egt_status spilled_tiles(egt_handle* h, int64_t* out) {
+    if (h->t_spilled < 0) {
+        unsigned long long v = 0;
+        EGT_CUDA_TRY(cudaMemcpyAsync(&v, h->d_counters + kCtrSpillTiles, sizeof(v), cudaMemcpyDeviceToHost, h->stream));
+        EGT_CUDA_TRY(cudaStreamSynchronize(h->stream));
+        h->t_spilled = (int64_t)v;
+    }
+    *out = h->t_spilled;
     return EGT_OK;
 }
 
@@ -852,10 +866,9 @@ static egt_status resident_loop(egt_handle* h, int iters, float lambda, float mu
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         const cudaError_t e = cudaLaunchKernelEx(
-            &cfg, k_taubin_resident, h->m_p, h->m_pb, (const int*)h->m_off, (const int*)h->m_col,
-            (const int*)h->t_uni, (const uint32_t*)h->t_loc, (const int*)h->t_nu, (const int*)h->t_soff,
-            (const uint32_t*)h->t_adj, adj_words(tiles), n, 2 * part, lambda, mu, h->taubin_tag, max_polls,
-            h->d_counters + kCtrTaubinFail);
+            &cfg, k_taubin_resident, h->m_p, h->m_pb, (const int*)h->m_off, (const int*)h->t_uni,
+            (const uint32_t*)h->t_loc, (const int*)h->t_nu, (const int*)h->t_soff, (const uint32_t*)h->t_adj,
+            adj_words(tiles), n, 2 * part, lambda, mu, h->taubin_tag, max_polls, h->d_counters + kCtrTaubinFail);
         if (*left == iters && (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported)) {
             cudaGetLastError();
             return EGT_OK;
@@ -912,7 +925,10 @@ egt_status run_taubin(egt_handle* h, int iters, float lambda, float mu) {
         }
         const unsigned blocks = wave[dev & 63].load();
         const int tiles = (n + kTile - 1) / kTile;
-        if (h->taubin_mode == 0 && h->t_adj && tiles <= (int)resident[dev & 63].load()) {
+        int64_t spilled = 1;
+        if (h->taubin_mode == 0 && h->t_adj && tiles <= (int)resident[dev & 63].load())
+            EGT_TRY(spilled_tiles(h, &spilled));
+        if (spilled == 0) {
             int left = 0;
             EGT_TRY(resident_loop(h, iters, lambda, mu, st, &left));
             if (left == 0) {
