@@ -253,7 +253,6 @@ struct DescArgs {
     float* kth;
     uint8_t* qlevel;
     unsigned long long* ctr;
-    bool jump;
 };
 
 __global__ void k_make_desc(DescArgs d, KnnArgs* __restrict__ out) {
@@ -283,7 +282,6 @@ __global__ void k_make_desc(DescArgs d, KnnArgs* __restrict__ out) {
     a.counters = d.ctr + (size_t)c * kCtrWords;
     a.maxpop = a.counters + kCtrMaxPop;
     a.gbase = o;
-    a.jump = d.jump;
     out[c] = a;
 }
 
@@ -335,7 +333,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_knn_batch(const KnnArgs* __rest
         for (int q = q0; q < q1; q++) {
             WarpList<S> L;
             bool invalid, rerun;
-            const int reached = plain_query<true, S>(a, np, q, a.p4[q], L, invalid, lane, s_pref[w], s_start[w],
+            const int reached = plain_query<true, S <= 2, S>(a, np, q, a.p4[q], L, invalid, lane, s_pref[w], s_start[w],
                                                      s_md[w], s_mp[w], rerun);
             write_query<S>(a, q, L, invalid, reached, lane);
             if (rerun && lane == 0) atomicAdd(&a.counters[kCtrExactRerun], 1ull);
@@ -376,7 +374,7 @@ __global__ void __launch_bounds__(kWarps * 32, 3) k_knn_egt_batch(const KnnArgs*
             const float4 pq = a.p4[q];
             WarpList<S> L;
             bool invalid, rerun;
-            const int reached = plain_query<true, S>(a, np, q, pq, L, invalid, lane, sc.pref, sc.start, sc.cd, sc.cj,
+            const int reached = plain_query<true, S <= 2, S>(a, np, q, pq, L, invalid, lane, sc.pref, sc.start, sc.cd, sc.cj,
                                                      rerun);
             write_query<S>(a, q, L, invalid, reached, lane);
             if (rerun && lane == 0) atomicAdd(&a.counters[kCtrExactRerun], 1ull);
@@ -523,7 +521,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_knn_list_batch(const KnnArgs* _
         const NormParams np = *a.np;
         WarpList<S> L;
         bool invalid, rerun;
-        const int reached = plain_query<true, S>(a, np, q, a.p4[q], L, invalid, lane, s_pref[w], s_start[w], s_md[w],
+        const int reached = plain_query<true, S <= 2, S>(a, np, q, a.p4[q], L, invalid, lane, s_pref[w], s_start[w], s_md[w],
                                                  s_mp[w], rerun);
         write_query<S>(a, q, L, invalid, reached, lane);
         if (rerun && lane == 0) atomicAdd(&a.counters[kCtrExactRerun], 1ull);
@@ -1024,7 +1022,6 @@ egt_status egt_batch_create(const float* xyz_host, const int64_t* offsets, const
     da.kth = h->kth;
     da.qlevel = h->qlevel;
     da.ctr = b->d_ctr;
-    da.jump = cfg.knn_mode != EGT_KNN_PLAIN;
     k_make_desc<<<blocks(count), kB, 0, st>>>(da, b->d_desc);
     BSTAT([&] { EGT_LAUNCH_CHECK(); return EGT_OK; }());
     k_maxpop_batch<<<dim3(kPopSlices, kMaxLevels, (unsigned)count), 256, 0, st>>>(b->d_desc);

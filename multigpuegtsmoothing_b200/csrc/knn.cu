@@ -43,7 +43,7 @@ namespace {
 // Persistent: one resident wave of blocks whose warps claim a.chunk queries at
 // a time, so that a warp that drew cheap queries moves on instead of idling
 // until the most expensive query of its block is done.
-template <int S, bool kFast>
+template <int S, bool kFast, bool kJump>
 __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_knn_plain(KnnArgs a) {
     __shared__ int s_pref[kWarps][32];
     __shared__ int s_start[kWarps][32];
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_knn_plain(KnnArgs a
             const float4 pq = a.p4[q];
             WarpList<S> L;
             bool invalid, rerun;
-            const int reached = plain_query<kFast, S>(a, np, q, pq, L, invalid, lane, s_pref[w], s_start[w], s_md[w],
+            const int reached = plain_query<kFast, kJump, S>(a, np, q, pq, L, invalid, lane, s_pref[w], s_start[w], s_md[w],
                                                       s_mp[w], rerun);
             write_query<S>(a, q, L, invalid, reached, lane);
             if (rerun && lane == 0) atomicAdd(&s_rerun, 1u);
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_knn_select(KnnArgs 
             }
             WarpList<S> L;
             bool invalid, rerun;
-            const int reached = plain_query<true, S>(a, np, q, pq, L, invalid, lane, sc.pref, sc.start, sc.cd, sc.cj,
+            const int reached = plain_query<true, false, S>(a, np, q, pq, L, invalid, lane, sc.pref, sc.start, sc.cd, sc.cj,
                                                      rerun);
             write_query<S>(a, q, L, invalid, reached, lane);
             __syncwarp();  // the scratch is rewritten by the next query
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_knn_learned(KnnArgs
             }
             if (!ok) {
                 bool rerun;
-                reached = plain_query<true, S>(a, np, q, pq, L, invalid, lane, s_pref[w], s_start[w], s_md[w],
+                reached = plain_query<true, S <= 2, S>(a, np, q, pq, L, invalid, lane, s_pref[w], s_start[w], s_md[w],
                                                s_mp[w], rerun);
                 if (rerun && lane == 0) atomicAdd(&s_rerun, 1u);
             }
@@ -576,7 +576,7 @@ __device__ __forceinline__ bool decide_query(const NormParams& np, int L, int o,
     return more;
 }
 
-template <bool kExact, int S>
+template <bool kExact, bool kJump, int S>
 __device__ int search_query(const KnnArgs& a, const NormParams& np, float4 pq, const float u[3], float thres_lt,
                             WarpList<S>& L, bool& invalid, int lane, int* s_pref, int* s_start, float* s_md,
                             int* s_mp) {
@@ -593,10 +593,10 @@ __device__ int search_query(const KnnArgs& a, const NormParams& np, float4 pq, c
     // list (first_full_level; no point is excluded here).
     int2 first = make_int2(-1, -1);
     int l1 = -1;
-    bool inside = !kExact && np.thres > 4.0f;
+    bool inside = kJump && np.thres > 4.0f;
 #pragma unroll
     for (int d = 0; d < 3; d++) inside = inside && u[d] >= 0.0f && u[d] < 1.0f;
-    if (inside) {
+    if (kJump && inside) {
         l1 = first_full_level(a, k, [&](int l) {
             const float B = (float)(1024 >> l);
             return make_int3((int)__fmul_rn(u[0], B), (int)__fmul_rn(u[1], B), (int)__fmul_rn(u[2], B));
@@ -604,14 +604,15 @@ __device__ int search_query(const KnnArgs& a, const NormParams& np, float4 pq, c
         if (l1 >= 0 && a.maxpop[l1] >= (unsigned long long)a.max_pts) l1 = -1;
     }
     cells(max(l1, 0));
-    if (l1 < 0) first = lane == 0 ? find_cell(a.lv[0], ci[0], ci[1], ci[2]) : make_int2(-1, -1);
-    stream_cells<kExact, S>(L, invalid, l1 < 0 ? 1 : 32, first.x, first.y, l1 < 0 ? nullptr : a.lv[l1].order, a.p4, -1,
-                            pq, thres_lt, l1 < 0 ? a.max_pts : INT_MAX, lane, -1, 0, 0, 0, s_pref, s_start, s_md,
-                            s_mp);
-    bool cont = decide_query(np, max(l1, 0), l1 < 0 ? 0 : 1, L.counter, k, kExact ? L.kth : L.fetch_dist(k - 1),
+    const bool own = !kJump || l1 < 0;
+    if (own) first = lane == 0 ? find_cell(a.lv[0], ci[0], ci[1], ci[2]) : make_int2(-1, -1);
+    stream_cells<kExact, S>(L, invalid, own ? 1 : 32, first.x, first.y, own ? nullptr : a.lv[max(l1, 0)].order, a.p4, -1,
+                            pq, thres_lt, own ? a.max_pts : INT_MAX, lane, -1, 0, 0, 0, s_pref, s_start, s_md, s_mp);
+    bool cont = decide_query(np, max(l1, 0), own ? 0 : 1, L.counter, k, kExact ? L.kth : L.fetch_dist(k - 1),
                              invalid, pq, ci);
     int reached = max(l1, 0);
-    for (int lvl = l1 + 1; cont && lvl < kMaxLevels; lvl++) {
+    for (int lvl = l1 + 1; cont; lvl++) {
+        if (kJump && lvl == kMaxLevels) break;  // a jump to the last level leaves none
         reached = lvl;
         const LevelDev& LV = a.lv[lvl];
 #pragma unroll
@@ -627,6 +628,7 @@ __device__ int search_query(const KnnArgs& a, const NormParams& np, float4 pq, c
         stream_cells<kExact, S>(L, invalid, 26, cell.x, cell.y, LV.order, a.p4, -1, pq, thres_lt, a.max_pts, lane,
                                 lvl - 1, cp[0], cp[1], cp[2], s_pref, s_start, s_md, s_mp, culled);
         cont = decide_query(np, lvl, 1, L.counter, k, kExact ? L.kth : L.fetch_dist(k - 1), invalid, pq, ci);
+        if (lvl == kMaxLevels - 1) break;
     }
     if (cont) { invalid = true; reached = kMaxLevels; }
     return reached;
@@ -635,7 +637,7 @@ __device__ int search_query(const KnnArgs& a, const NormParams& np, float4 pq, c
 // qpos: normalised query positions; query j (processing order a.qmap[j]) is
 // row a.qmap[j] of out, in original reference ids (perm), -1 padded; an
 // invalid query's row is all -1 (negateNotValidKnnIndexes, :291-302).
-template <int S>
+template <int S, bool kJump>
 __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_knn_query(KnnArgs a, const float4* __restrict__ qpos,
                                                                      const int* __restrict__ perm,
                                                                      int* __restrict__ out) {
@@ -658,10 +660,10 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_knn_query(KnnArgs a
                                 __fdiv_rn(__fsub_rn(pq.z, np.a), ab)};
             WarpList<S> L;
             bool invalid;
-            search_query<false, S>(a, np, pq, u, thres_lt, L, invalid, lane, s_pref[w], s_start[w], s_md[w], s_mp[w]);
+            search_query<false, kJump, S>(a, np, pq, u, thres_lt, L, invalid, lane, s_pref[w], s_start[w], s_md[w], s_mp[w]);
             if (has_ties(L, min(L.counter, a.k + 1), lane)) {
-                search_query<true, S>(a, np, pq, u, thres_lt, L, invalid, lane, s_pref[w], s_start[w], s_md[w],
-                                      s_mp[w]);
+                search_query<true, false, S>(a, np, pq, u, thres_lt, L, invalid, lane, s_pref[w], s_start[w],
+                                             s_md[w], s_mp[w]);
                 if (lane == 0) atomicAdd(&a.counters[kCtrExactRerun], 1ull);
             }
 #pragma unroll
@@ -742,11 +744,20 @@ egt_status launch_learned(const KnnArgs& a, const uint8_t* cls, cudaStream_t st)
     return EGT_OK;
 }
 
-template <int S, bool kFast>
-egt_status launch(const KnnArgs& a, cudaStream_t st) {
+template <int S, bool kFast, bool kJump>
+egt_status launch_plain(const KnnArgs& a, cudaStream_t st) {
     unsigned G = 0;
-    EGT_TRY(wave_blocks(k_knn_plain<S, kFast>, a.n, &G));
-    return launch_dependent(k_knn_plain<S, kFast>, dim3(G), dim3(kWarps * 32), 0, st, a);
+    EGT_TRY(wave_blocks(k_knn_plain<S, kFast, kJump>, a.n, &G));
+    return launch_dependent(k_knn_plain<S, kFast, kJump>, dim3(G), dim3(kWarps * 32), 0, st, a);
+}
+
+// queries: how many the search is about (kWalk: never jump).
+constexpr int64_t kWalk = -1;
+template <int S>
+egt_status launch(const KnnArgs& a, int64_t queries, cudaStream_t st) {
+    if constexpr (S <= 3)
+        if (queries != kWalk && jump_pays<S>(queries, a.k)) return launch_plain<S, true, true>(a, st);
+    return launch_plain<S, true, false>(a, st);
 }
 
 }  // namespace
@@ -778,22 +789,25 @@ static egt_status knn_prepare(egt_handle* h, int k, KnnArgs* a) {
     a->counters = h->d_counters;
     a->maxpop = h->d_counters + kCtrMaxPop;
     a->qmap = nullptr;
-    a->jump = h->cfg.knn_mode != EGT_KNN_PLAIN;
     return EGT_OK;
 }
 
-// One plain search launch over a.n queries (the work counter must be zero).
-static egt_status knn_launch(const KnnArgs& a, cudaStream_t st) {
+// One plain search launch over a.n queries, of a search of `queries` (the work
+// counter must be zero).
+static egt_status knn_launch(const KnnArgs& a, int64_t queries, cudaStream_t st) {
     const int k = a.k;
     // the list keeps k+1 slots (k for k = 256, which always uses the exact rule)
-    if (k + 1 <= 32) EGT_TRY((launch<1, true>(a, st)));
-    else if (k + 1 <= 64) EGT_TRY((launch<2, true>(a, st)));
-    else if (k + 1 <= 96) EGT_TRY((launch<3, true>(a, st)));
-    else if (k + 1 <= 128) EGT_TRY((launch<4, true>(a, st)));
-    else if (k + 1 <= 256) EGT_TRY((launch<8, true>(a, st)));
-    else EGT_TRY((launch<8, false>(a, st)));
-    return EGT_OK;
+    if (k + 1 <= 32) return launch<1>(a, queries, st);
+    if (k + 1 <= 64) return launch<2>(a, queries, st);
+    if (k + 1 <= 96) return launch<3>(a, queries, st);
+    if (k + 1 <= 128) return launch<4>(a, queries, st);
+    if (k + 1 <= 256) return launch<8>(a, queries, st);
+    return launch_plain<8, false, false>(a, st);
 }
+
+// The queries an unqualified search of h counts: EGT_KNN_PLAIN is the
+// reference's schedule and takes its steps one by one.
+static int64_t jump_queries(const egt_handle* h) { return h->cfg.knn_mode == EGT_KNN_PLAIN ? kWalk : h->n; }
 
 template <typename K>
 static egt_status select_blocks(K kernel, unsigned* out) {
@@ -835,8 +849,8 @@ static egt_status launch_select(const KnnArgs& a, cudaStream_t st) {
 // reference's ring search (k_knn_plain), or with `select` (EGT_KNN_SELECT, k <=
 // kSelMaxK) the block-selection kernel, whose uncertified queries run the ring
 // search in the same launch.
-static egt_status knn_search(const KnnArgs& a, bool select, cudaStream_t st) {
-    if (!select || a.k > kSelMaxK) return knn_launch(a, st);
+static egt_status knn_search(const KnnArgs& a, bool select, int64_t queries, cudaStream_t st) {
+    if (!select || a.k > kSelMaxK) return knn_launch(a, queries, st);
     KnnArgs as = a;
     as.chunk = kSelChunk;
     if (a.k + 1 <= 32) return launch_select<1>(as, st);
@@ -857,7 +871,7 @@ static egt_status tile_search(egt_handle* h, const KnnArgs& a, cudaStream_t st) 
     ar.qmap = t.ring2;
     ar.n_dev = t.n_ring2;
     ar.work = h->d_counters + kCtrTileRingWork;
-    return knn_launch(ar, st);
+    return knn_launch(ar, 0, st);  // few
 }
 
 // Whether EGT_KNN_TILE takes the cell-tile search.
@@ -872,7 +886,7 @@ egt_status run_knn(egt_handle* h, int k) {
     const bool tile = h->cfg.knn_mode == EGT_KNN_TILE;
     h->knn_untiled = tile && k >= kTileLowK && k <= kTileMaxK && !tile_takes(h->n, k);
     if (tile && tile_takes(h->n, k)) EGT_TRY(tile_search(h, a, st));
-    else EGT_TRY(knn_search(a, h->cfg.knn_mode == EGT_KNN_SELECT, st));
+    else EGT_TRY(knn_search(a, h->cfg.knn_mode == EGT_KNN_SELECT, jump_queries(h), st));
     EGT_CUDA_TRY(cudaEventRecord(h->ev[3], st));
     return EGT_OK;
 }
@@ -998,7 +1012,7 @@ egt_status run_knn_host(egt_handle* h, int k, int* host) {
         ac.n = m;
         ac.work = work + c;
         ac.n_ring = work + chunks + c;
-        s = knn_search(ac, h->cfg.knn_mode == EGT_KNN_SELECT, cs);
+        s = knn_search(ac, h->cfg.knn_mode == EGT_KNN_SELECT, jump_queries(h), cs);
         if (s != EGT_OK) break;
         const int64_t cnt = (int64_t)m * k;
         k_rows_original<<<(unsigned)((cnt + T - 1) / T), T, 0, cs>>>(h->lists, h->perm, qmap + r0, m, k, out);
@@ -1032,11 +1046,16 @@ egt_status run_knn_host(egt_handle* h, int k, int* host) {
     return s;
 }
 
-template <int S>
+// Queries jump with lists of one register a lane, from k = 3 (fewer neighbours are
+// often in the query's own cell; longer lists: see kJumpEntries).  Against 1M
+// points, 100,000 queries: k = 1 0.87 times as fast with the jump, 2 0.96, 4 1.03, 8
+// 1.08, 31 1.04, 50 0.92, 80 0.85, 128 0.80.
+constexpr int kQueryJumpK = 3;
+template <int S, bool kJump>
 static egt_status launch_query(const KnnArgs& a, const float4* qpos, const int* perm, int* out, cudaStream_t st) {
     unsigned G = 0;
-    EGT_TRY(wave_blocks(k_knn_query<S>, a.n, &G));
-    k_knn_query<S><<<G, kWarps * 32, 0, st>>>(a, qpos, perm, out);
+    EGT_TRY(wave_blocks(k_knn_query<S, kJump>, a.n, &G));
+    k_knn_query<S, kJump><<<G, kWarps * 32, 0, st>>>(a, qpos, perm, out);
     EGT_LAUNCH_CHECK();
     return EGT_OK;
 }
@@ -1097,11 +1116,12 @@ egt_status run_knn_query(egt_handle* h, const float* q_host, int64_t nq, int k, 
     a.maxpop = h->d_counters + kCtrMaxPop;
     a.qmap = qmap;
     egt_status s;
-    if (k + 1 <= 32) s = launch_query<1>(a, qpos, h->perm, out, st);
-    else if (k + 1 <= 64) s = launch_query<2>(a, qpos, h->perm, out, st);
-    else if (k + 1 <= 96) s = launch_query<3>(a, qpos, h->perm, out, st);
-    else if (k + 1 <= 128) s = launch_query<4>(a, qpos, h->perm, out, st);
-    else s = launch_query<8>(a, qpos, h->perm, out, st);
+    if (k + 1 <= 32 && k >= kQueryJumpK) s = launch_query<1, true>(a, qpos, h->perm, out, st);
+    else if (k + 1 <= 32) s = launch_query<1, false>(a, qpos, h->perm, out, st);
+    else if (k + 1 <= 64) s = launch_query<2, false>(a, qpos, h->perm, out, st);
+    else if (k + 1 <= 96) s = launch_query<3, false>(a, qpos, h->perm, out, st);
+    else if (k + 1 <= 128) s = launch_query<4, false>(a, qpos, h->perm, out, st);
+    else s = launch_query<8, false>(a, qpos, h->perm, out, st);
     unsigned long long inv = 0;
     if (s == EGT_OK) {
         cudaError_t e = cudaMemcpyAsync(out_host, out, sizeof(int) * (size_t)n * k, cudaMemcpyDeviceToHost, st);

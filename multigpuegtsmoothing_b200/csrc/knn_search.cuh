@@ -21,10 +21,6 @@ struct KnnArgs {
     uint8_t* __restrict__ qlevel;
     unsigned long long* __restrict__ counters;
     const unsigned long long* __restrict__ maxpop = nullptr;  // [kMaxLevels] largest cell population of each level
-    // The search may start at the first level that can fill the list
-    // (first_full_level).  Off for EGT_KNN_PLAIN, which takes the reference's
-    // steps one by one: the other modes' speed is judged against it.
-    bool jump = true;
     const int* __restrict__ qmap = nullptr;  // query j of a launch is qmap[j] (nullptr: j)
     unsigned long long* __restrict__ work = nullptr;  // work counter (nullptr: counters[kCtrWork])
     const unsigned long long* __restrict__ n_dev = nullptr;  // launch size on the device (nullptr: n)
@@ -297,16 +293,33 @@ __device__ __forceinline__ int first_full_level(const KnnArgs& a, int need, CI&&
     return -1;
 }
 
+// The ring search jumps (first_full_level) with lists of one or two registers a
+// lane, with three in launches of up to kJumpEntries list entries (queries times
+// k+1), and with more never: a list that fills late gains little over the walk,
+// whose cells are culled once the list is full, and the jump's live values spill
+// beside a long list.  Time without the jump over time with it: superquadrics, k =
+// 90, 20,000 points 1.07, 100,000 1.05, 300,000 1.01; eight clusters of widths 0.002
+// to 0.3, k = 90, 0.94, 0.98, 0.96 (to 75,000 points still ahead of the walk with
+// four queries to a claim); k = 110: 1.02 and 0.87 at 20,000, 0.89 and 0.91 at
+// 300,000; k = 200: 0.89 and 0.81, 0.82 and 0.88.
+constexpr int64_t kJumpEntries = int64_t(1) << 23;
+template <int S>
+inline bool jump_pays(int64_t queries, int k) {
+    return S <= 2 || queries * (k + 1) <= kJumpEntries;
+}
+
 // The whole reference search for query q.  Returns the level reached
 // (kMaxLevels when the query ran out of levels).  kExact keeps the k-slot
 // list of the reference's insertion rule; otherwise the list keeps k+1 slots
 // (one more than the output) so that has_ties can check the k-th/(k+1)-th
-// boundary, and the steps that cannot fill the list are taken as one
-// (first_full_level).  Either way the decisions see the k-th smallest distance
-// offered so far, which does not depend on the insertion rule.
-template <bool kExact, int S>
+// boundary.  Either way the decisions see the k-th smallest distance offered so
+// far, which does not depend on the insertion rule.  kJump (not with kExact): the
+// steps that cannot fill the list are taken as one (first_full_level); a template
+// parameter, so that the walk alone keeps its registers.
+template <bool kExact, bool kJump, int S>
 __device__ int search(const KnnArgs& a, const NormParams& np, int q, float4 pq, WarpList<S>& L,
                       bool& invalid, int lane, int* s_pref, int* s_start, float* s_md, int* s_mp) {
+    static_assert(!(kExact && kJump), "the exact rule sees every step");
     const uint32_t c0 = __float_as_uint(pq.w);
     const int cx0 = c0 & 1023, cy0 = (c0 >> 10) & 1023, cz0 = (c0 >> 20) & 1023;
     const int k = a.k;
@@ -314,19 +327,20 @@ __device__ int search(const KnnArgs& a, const NormParams& np, int q, float4 pq, 
     invalid = false;
     int2 first = make_int2(-1, -1);
     int l1 = -1;  // the level to start at (-1: the query's own level-0 cell)
-    if (!kExact && a.jump && np.thres > 4.0f) {
+    if (kJump && np.thres > 4.0f) {
         l1 = first_full_level(a, k + 1, [&](int l) { return make_int3(cx0 >> l, cy0 >> l, cz0 >> l); }, lane, first);
         if (l1 >= 0 && a.maxpop[l1] >= (unsigned long long)a.max_pts) l1 = -1;  // populations grow with the level
     }
     // offset 0 at level 0: the query's own cell (always occupied)
-    if (l1 < 0) first = lane == 0 ? find_cell(a.lv[0], cx0, cy0, cz0) : make_int2(-1, -1);
-    stream_cells<kExact, S>(L, invalid, l1 < 0 ? 1 : 32, first.x, first.y, l1 < 0 ? nullptr : a.lv[l1].order, a.p4, q,
-                            pq, np.thres, l1 < 0 ? a.max_pts : INT_MAX, lane, -1, 0, 0, 0, s_pref, s_start, s_md,
-                            s_mp);
-    bool cont = decide(np, max(l1, 0), l1 < 0 ? 0 : 1, L.counter, k, kExact ? L.kth : L.fetch_dist(k - 1), invalid, pq,
+    if (!kJump || l1 < 0) first = lane == 0 ? find_cell(a.lv[0], cx0, cy0, cz0) : make_int2(-1, -1);
+    const bool own = !kJump || l1 < 0;
+    stream_cells<kExact, S>(L, invalid, own ? 1 : 32, first.x, first.y, own ? nullptr : a.lv[max(l1, 0)].order, a.p4, q,
+                            pq, np.thres, own ? a.max_pts : INT_MAX, lane, -1, 0, 0, 0, s_pref, s_start, s_md, s_mp);
+    bool cont = decide(np, max(l1, 0), own ? 0 : 1, L.counter, k, kExact ? L.kth : L.fetch_dist(k - 1), invalid, pq,
                        cx0, cy0, cz0);
     int reached = max(l1, 0);
-    for (int lvl = l1 + 1; cont && lvl < kMaxLevels; lvl++) {
+    for (int lvl = l1 + 1; cont; lvl++) {
+        if (kJump && lvl == kMaxLevels) break;  // a jump to the last level leaves none
         reached = lvl;
         const LevelDev& LV = a.lv[lvl];
         int2 cell = make_int2(-1, -1);
@@ -341,6 +355,7 @@ __device__ int search(const KnnArgs& a, const NormParams& np, int q, float4 pq, 
         stream_cells<kExact, S>(L, invalid, 26, cell.x, cell.y, LV.order, a.p4, q, pq, np.thres, a.max_pts, lane,
                                 lvl - 1, cx0 >> sL, cy0 >> sL, cz0 >> sL, s_pref, s_start, s_md, s_mp, culled);
         cont = decide(np, lvl, 1, L.counter, k, kExact ? L.kth : L.fetch_dist(k - 1), invalid, pq, cx0, cy0, cz0);
+        if (lvl == kMaxLevels - 1) break;
     }
     // still searching after the B = 8 ring: invalid (GridKNNCuda.cu:2572-2586)
     if (cont) { invalid = true; reached = kMaxLevels; }
@@ -350,17 +365,17 @@ __device__ int search(const KnnArgs& a, const NormParams& np, int q, float4 pq, 
 // One query of the plain search: the fast list rule first; if the k+1 kept
 // distances are not pairwise distinct the order of equal distances matters
 // and the query is searched again with the reference's exact rule.
-template <bool kFast, int S>
+template <bool kFast, bool kJump, int S>
 __device__ __forceinline__ int plain_query(const KnnArgs& a, const NormParams& np, int q, float4 pq, WarpList<S>& L,
                                            bool& invalid, int lane, int* s_pref, int* s_start, float* s_md,
                                            int* s_mp, bool& rerun) {
     rerun = false;
     if (kFast) {
-        const int reached = search<false, S>(a, np, q, pq, L, invalid, lane, s_pref, s_start, s_md, s_mp);
+        const int reached = search<false, kJump, S>(a, np, q, pq, L, invalid, lane, s_pref, s_start, s_md, s_mp);
         if (!has_ties(L, min(L.counter, a.k + 1), lane)) return reached;
         rerun = true;
     }
-    return search<true, S>(a, np, q, pq, L, invalid, lane, s_pref, s_start, s_md, s_mp);
+    return search<true, false, S>(a, np, q, pq, L, invalid, lane, s_pref, s_start, s_md, s_mp);
 }
 
 // Writes the outputs of query q from its final list.

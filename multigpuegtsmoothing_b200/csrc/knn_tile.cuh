@@ -666,8 +666,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, Form::kWarps) k_knn_tile(KnnA
         const NormParams np = *A.np;
         WarpList<S> L;
         bool invalid, rerun;
-        const int reached = plain_query<true, S>(A, np, q, A.p4[q], L, invalid, lane, r_pref, r_start, r_md, r_mp,
-                                                 rerun);
+        const int reached = plain_query<true, true, S>(A, np, q, A.p4[q], L, invalid, lane, r_pref, r_start, r_md,
+                                                       r_mp, rerun);
         write_query<S>(A, q, L, invalid, reached, lane);
         if constexpr (kBatch) {
             if (rerun && lane == 0) atomicAdd(&A.counters[kCtrExactRerun], 1ull);
