@@ -48,7 +48,7 @@ typedef struct egt_proposal egt_proposal;
 #define EGT_KNN_SELECT 2   /* block selection, certified rows; the ring search for the rest */
 #define EGT_KNN_TILE 3     /* cell tiles (default): a cell's queries one per lane over its 3x3x3
                               block, certified rows; the ring search for the rest.  For 16 <= k <= 64
-                              and at least 50,000 points, and 8 <= k <= 15 and at least 65,536; other
+                              and at least 40,000 points, and 8 <= k <= 15 and at least 100,000; other
                               k and smaller clouds use the ring search */
 
 /* Tunables.  Defaults reproduce the reference CLI (main.cpp:108-116). */

@@ -1,5 +1,6 @@
 // C ABI of libegt_b200 (declared in include/egt_b200.h): handle lifecycle,
 // argument checking, error reporting and the stage entry points.
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -544,7 +545,7 @@ egt_status egt_get_timings(egt_handle* h, egt_timings* t) {
     h->tm.exact_reruns = (int64_t)ctr[kCtrExactRerun];
     h->tm.knn_fallback = h->last_knn_learned ? 0
                          : h->knn_untiled    ? h->n
-                                             : (int64_t)(ctr[kCtrSelFallback] + ctr[kCtrTileRing2]);
+                                             : std::min(h->n, (int64_t)(ctr[kCtrSelFallback] + ctr[kCtrTileRing2]));
     h->tm.knn_evaluations = h->last_knn_learned ? 0 : (int64_t)ctr[kCtrEvals];
     h->tm.egt_tests = (int64_t)ctr[kCtrEgtTests];
     h->tm.taubin_spill_tiles = h->tm.taubin_tiles > 0 ? (int64_t)ctr[kCtrSpillTiles] : 0;

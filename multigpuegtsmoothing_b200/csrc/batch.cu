@@ -632,7 +632,8 @@ egt_status knn_batch(egt_batch* b) {
     if (tile) {
         tile = false;
         // (the batch's points share the launches: their total decides)
-        for (int c = 0; c < b->count; c++) tile |= tile_takes(b->N, b->k[c]);
+        for (int c = 0; c < b->count; c++)
+            tile |= tile_takes(b->N, b->k[c]) && (b->k[c] >= kTileLowK || b->N >= kTileMinCloudLowK * b->count);
     }
     if (tile) {
         if (kk + 1 <= 32) EGT_TRY(knn_batch_tile<1>(b, st));

@@ -65,13 +65,20 @@ constexpr int kTilePosBits = 13;  // block positions (kTileMaxBlock)
 constexpr int kTileMaxUnsorted = 16;  // points below the bucket range a query may have (more: the ring search)
 // Smallest k and cloud the tile search takes.  Below kTileMinPoints points its
 // chain of launches and its long batches cost more than the ring search of
-// every query (k = 40: 8K points 151 against 53 us, 36K 217 against 168; 72K 274
-// against 304); k of 8 to 15 pays from kTileMinPointsLowK points (k = 10: 36K
-// points 131 against 136 us, 72K 150 against 248, 1M 1.95 against 2.60 ms).
+// every query (sphere, k = 16: 30,000 points 97 against 94 us, 40,000 126 against
+// 139, 50,000 140 against 191; clustered clouds turn later, 100,000 to 200,000, but
+// there the tiles are still 1.2 to 1.5 times as fast as with 16 warps and
+// insertion sorts); k of 8 to 15 pays from kTileMinPointsLowK points
+// (superquadrics, k = 8: 65,536 points 0.65 times the ring search's speed, 100,000
+// 0.74, 200,000 1.05, 1M 1.8; sphere 1.7, 1.8, 1.8, 1.9), and not where more than one
+// query in kTileLowShare is left to the ring search (k_tile_gather).
 constexpr int kTileMinK = 8;
 constexpr int kTileLowK = 16;
-constexpr int64_t kTileMinPoints = 50000;
-constexpr int64_t kTileMinPointsLowK = 65536;
+constexpr int64_t kTileMinPoints = 40000;
+constexpr int64_t kTileMinPointsLowK = 100000;
+constexpr int kTileLowShare = 16;
+constexpr int64_t kTileMinCloudLowK = 5000;  // points a cloud in a batch, on average (k = 10: 64 clouds of 2,000 points
+                                             // 503 against 444 us, 10 of 12,000 273 against 369)
 constexpr int kTileMaxK = 64;    // largest k the cell-tile search takes
 inline bool tile_takes(int64_t n, int k) {
     return k >= kTileMinK && k <= kTileMaxK && n >= (k < kTileLowK ? kTileMinPointsLowK : kTileMinPoints);
@@ -116,6 +123,7 @@ struct TileArgs {
     const KnnArgs* desc;
     const uint16_t* cloud_of;
     int npts;                         // points of all clouds
+    bool low_k;                       // every k the tiles take is below kTileLowK
 };
 
 // The search arguments of cloud c: the kernel's own (one cloud), or the
@@ -269,6 +277,16 @@ __device__ __forceinline__ int tile_class(int pop) {
     return pop >= 4096 ? 0 : pop >= 2048 ? 1 : pop >= 1024 ? 2 : pop >= 512 ? 3 : pop >= 256 ? 4 : 5;
 }
 
+// Whether the search leaves every query to the launch after the tile kernel:
+// with k below kTileLowK, when the assignment left more than one query in
+// kTileLowShare to the ring search.  Short lists make the ring search cheap and
+// the dense blocks of such clouds dear: eight clusters of widths 0.002 to 0.3, k = 8,
+// 13 % left: 100,000 points 0.81 times the ring search's speed with tiles;
+// 62 %: 1M 0.60.
+__device__ __forceinline__ bool tile_bails(const TileArgs& t) {
+    return t.low_k && *t.n_ring * kTileLowShare > (unsigned long long)t.npts;
+}
+
 // Per unit (one warp per unit, grid-stride): its query count and block class,
 // and the batch count of each class.
 template <bool kBatch>
@@ -278,6 +296,7 @@ __global__ void __launch_bounds__(256) k_tile_count(KnnArgs a, TileArgs t) {
     const int lane = threadIdx.x & 31;
     const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nw = (int)((gridDim.x * blockDim.x) >> 5);
+    if (tile_bails(t)) return;
     const unsigned long long nu = *t.n_units;
     for (unsigned long long u = gw; u < nu; u += nw) {
         int c, l, ci;
@@ -323,6 +342,12 @@ __global__ void __launch_bounds__(256) k_tile_gather(KnnArgs a, TileArgs t) {
     const int lane = threadIdx.x & 31;
     const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nw = (int)((gridDim.x * blockDim.x) >> 5);
+    if (tile_bails(t)) {
+        for (int i = (int)(blockIdx.x * blockDim.x + threadIdx.x); i < t.npts; i += (int)(gridDim.x * blockDim.x))
+            t.ring2[i] = i;
+        if (blockIdx.x == 0 && threadIdx.x == 0) *t.n_ring2 = (unsigned long long)t.npts;
+        return;
+    }
     const unsigned long long nu = *t.n_units;
     // first batch of each class
     unsigned long long coff = 0;
@@ -637,6 +662,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, Form::kWarps) k_knn_tile(KnnA
     extern __shared__ __align__(16) unsigned char s_tile[];
     grid_dependency_wait();
     grid_dependents_launch();
+    if (tile_bails(t)) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int hl = lane & 15, hf = lane >> 4;
     unsigned char* base = s_tile + (size_t)w * kWarpBytes;
@@ -1002,7 +1028,8 @@ egt_status tile_kernel_launch(const KnnArgs& a, const TileArgs& t, cudaStream_t 
 
 // kmax: the largest k among the queries the tile search takes.
 template <bool kBatch>
-egt_status tile_launch(const KnnArgs& a, const TileArgs& t, int kmax, cudaStream_t st) {
+egt_status tile_launch(const KnnArgs& a, TileArgs t, int kmax, cudaStream_t st) {
+    t.low_k = kmax < kTileLowK;
     const unsigned T = 256;
     const int64_t npts = t.npts;
     EGT_TRY(launch_dependent(k_tile_assign<kBatch>, dim3((unsigned)((npts + T - 1) / T)), dim3(T), 0, st, a, t));
