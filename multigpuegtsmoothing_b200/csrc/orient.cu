@@ -31,6 +31,7 @@
 #include <numeric>
 #include <vector>
 #include "egt_internal.cuh"
+#include "radix.cuh"
 
 namespace egt {
 namespace {
@@ -50,11 +51,14 @@ __device__ __forceinline__ void block_count(unsigned long long* ctr, bool pred) 
 // Every edge {u, v}, u < v, belongs to the bucket of u.  Row u's own entries
 // above u go there directly; an entry u of a row v > u only if row u does not
 // list v (most do, so few entries need an atomic).  A bucket is then ordered
-// by v (rank by counting, buckets are short) and repeated entries dropped, which
-// puts the edges in (u, v) order: the reference's key order, without sorting
-// 64-bit keys (1M points, 16M list entries: 1.03 ms with a radix sort).
+// by v and repeated entries dropped, which puts the edges in (u, v) order: the
+// reference's key order, without sorting 64-bit keys (1M points, 16M list entries:
+// 1.03 ms with a radix sort).  The order comes from counting, quadratic in a
+// bucket, whose length is the rows that list u; buckets of more than kLongBucket
+// entries (equal points all list the same few of them) are sorted first.
 
 constexpr int kRowLanes = 16;  // lanes per row
+constexpr int kLongBucket = 1024;
 
 // keep[e]: 1 = bucket of its own row, 2 = bucket of the other end.  own[i]:
 // entries of kind 1; cnt[u]: entries of bucket u (zero before).
@@ -89,16 +93,18 @@ __global__ void __launch_bounds__(kTB) k_bucket_count(const int* __restrict__ of
 }
 
 // Fills the buckets (boff: their starts).  own[u] becomes bucket u's next free
-// place after its own row's entries.
+// place after its own row's entries.  longs [*n_long]: the buckets to sort.
 __global__ void __launch_bounds__(kTB) k_bucket_fill(const int* __restrict__ off, const int* __restrict__ col, int n,
                                                      int bits, const unsigned char* __restrict__ keep,
                                                      const int* __restrict__ boff, int* __restrict__ own,
-                                                     unsigned long long* __restrict__ key) {
+                                                     unsigned long long* __restrict__ key, int* __restrict__ longs,
+                                                     int* __restrict__ n_long) {
     const int i = (int)((blockIdx.x * (int64_t)kTB + threadIdx.x) / kRowLanes);
     const int l = threadIdx.x & (kRowLanes - 1);
     const int e0 = i < n ? off[i] : 0, e1 = i < n ? off[i + 1] : 0;
     const unsigned gmask = 0xffffu << (threadIdx.x & 16);
     int at = i < n ? boff[i] : 0;
+    if (l == 0 && i < n && boff[i + 1] - at > kLongBucket) longs[atomicAdd(n_long, 1)] = i;
     const int rounds = (e1 - e0 + kRowLanes - 1) / kRowLanes;
     for (int r = 0; r < rounds; r++) {  // uniform over the row's lanes
         const int e = e0 + r * kRowLanes + l;
@@ -113,6 +119,79 @@ __global__ void __launch_bounds__(kTB) k_bucket_fill(const int* __restrict__ off
             }
         }
         at += __popc(b);
+    }
+}
+
+// Sorts the long buckets by v, a block per bucket: least-significant-digit passes
+// between key and tmp (the same places), digits of 8 bits, the last pass ending in
+// key.  A pass takes the bucket in chunks and keeps each digit's next place.
+// 200,000 points, 50,000 of them equal, orientation: k = 16 23.1 ms by counting
+// alone, 2.0 with a sort of all keys, 0.99 so; k = 40 54.5, 3.5 and 1.44.
+constexpr int kSortItems = 8;
+__global__ void __launch_bounds__(kRadixThreads) k_bucket_sort(unsigned long long* key, unsigned long long* tmp,
+                                                               const int* __restrict__ boff,
+                                                               const int* __restrict__ longs,
+                                                               const int* __restrict__ n_long, int bits) {
+    __shared__ uint16_t s_cnt[kRadixWarps][kRadixBins];  // digits seen by each warp, then the warps' offsets
+    __shared__ uint32_t s_next[kRadixBins];              // next place of each digit
+    __shared__ uint32_t s_scan[kRadixWarps];
+    constexpr int kChunk = kRadixThreads * kSortItems;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, d = threadIdx.x;
+    for (int b = blockIdx.x; b < *n_long; b += gridDim.x) {
+        const int b0 = boff[longs[b]], m = boff[longs[b] + 1] - b0;
+        unsigned long long *src = key + b0, *dst = tmp + b0;
+        for (int shift = 0; shift < bits; shift += kRadixBits) {
+            s_next[d] = 0u;
+            __syncthreads();
+            for (int i = threadIdx.x; i < m; i += kRadixThreads)
+                atomicAdd(&s_next[(uint32_t)(src[i] >> shift) & (kRadixBins - 1u)], 1u);
+            __syncthreads();
+            const uint32_t base = radix_block_prefix(s_next[d], s_scan);
+            s_next[d] = base;
+            for (int c0 = 0; c0 < m; c0 += kChunk) {
+                for (int i = threadIdx.x; i < kRadixWarps * kRadixBins / 2; i += kRadixThreads)
+                    reinterpret_cast<uint32_t*>(&s_cnt[0][0])[i] = 0u;
+                __syncthreads();
+                unsigned long long k[kSortItems];
+                uint32_t rank[kSortItems];
+                const int at0 = c0 + w * 32 * kSortItems + lane;
+#pragma unroll
+                for (int i = 0; i < kSortItems; i++) k[i] = at0 + 32 * i < m ? src[at0 + 32 * i] : 0ull;
+#pragma unroll
+                for (int i = 0; i < kSortItems; i++) {
+                    const bool valid = at0 + 32 * i < m;
+                    const uint32_t e = (uint32_t)(k[i] >> shift) & (kRadixBins - 1u);
+                    const unsigned peers = radix_peers(e, valid);
+                    rank[i] = s_cnt[w][e] + __popc(peers & ((1u << lane) - 1u));
+                    __syncwarp();
+                    if (valid && (peers >> lane) == 1u) s_cnt[w][e] = (uint16_t)(rank[i] + 1);  // the last of its peers
+                    __syncwarp();
+                }
+                __syncthreads();
+                uint32_t tot = 0;
+#pragma unroll
+                for (int u = 0; u < kRadixWarps; u++) {
+                    const uint32_t c = s_cnt[u][d];
+                    s_cnt[u][d] = (uint16_t)tot;
+                    tot += c;
+                }
+                __syncthreads();
+#pragma unroll
+                for (int i = 0; i < kSortItems; i++) {
+                    const uint32_t e = (uint32_t)(k[i] >> shift) & (kRadixBins - 1u);
+                    if (at0 + 32 * i < m) dst[s_next[e] + s_cnt[w][e] + rank[i]] = k[i];
+                }
+                __syncthreads();
+                s_next[d] += tot;
+            }
+            __syncthreads();  // the pass is written before the next one reads it
+            unsigned long long* t = src;
+            src = dst;
+            dst = t;
+        }
+        if (src != key + b0)
+            for (int i = threadIdx.x; i < m; i += kRadixThreads) dst[i] = src[i];
+        __syncthreads();
     }
 }
 
@@ -133,10 +212,15 @@ __global__ void __launch_bounds__(kTB) k_bucket_edges(const unsigned long long* 
     const int b0 = boff[u], b1 = boff[u + 1];
     int p = b0;
     bool again = false;
-    for (int f = b0; f < b1; f++) {
-        const unsigned long long o = key[f];
-        p += (o < k || (o == k && f < e)) ? 1 : 0;
-        again |= o == k && f < e;
+    if (b1 - b0 > kLongBucket) {  // sorted (k_bucket_sort)
+        p = (int)e;
+        again = e > b0 && key[e - 1] == k;
+    } else {
+        for (int f = b0; f < b1; f++) {
+            const unsigned long long o = key[f];
+            p += (o < k || (o == k && f < e)) ? 1 : 0;
+            again |= o == k && f < e;
+        }
     }
     ukey[p] = k;
     if (again) { act[p] = kNone; return; }
@@ -542,8 +626,9 @@ egt_status run_orient(egt_handle* h) {
     auto take = [&](size_t bytes) { const size_t a = at; at += (bytes + 255) & ~(size_t)255; return a; };
     const size_t o_key = take(sizeof(unsigned long long) * nnz), o_ukey = take(sizeof(unsigned long long) * nnz),
                  o_act = take(sizeof(unsigned long long) * nnz), o_sgn = take(nnz), o_keep = take(nnz),
-                 o_cnt = take(sizeof(int) * (n + 1)), o_boff = take(sizeof(int) * (n + 1)),
-                 o_own = take(sizeof(int) * n), o_scan = take(t_scan);
+                 o_cnt = take(sizeof(int) * (n + 2)), o_boff = take(sizeof(int) * (n + 1)),
+                 o_own = take(sizeof(int) * n), o_scan = take(t_scan),
+                 o_longs = take(sizeof(int) * (nnz / kLongBucket + 1));
     char* m = nullptr;
     EGT_CUDA_TRY(cudaMallocAsync((void**)&m, at, st));
     auto* key = reinterpret_cast<unsigned long long*>(m + o_key);
@@ -554,12 +639,20 @@ egt_status run_orient(egt_handle* h) {
     auto* cnt = reinterpret_cast<int*>(m + o_cnt);
     auto* boff = reinterpret_cast<int*>(m + o_boff);
     auto* own = reinterpret_cast<int*>(m + o_own);
-    EGT_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int) * (n + 1), st));
+    auto* longs = reinterpret_cast<int*>(m + o_longs);
+    int* n_long = cnt + n + 1;
+    EGT_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int) * (n + 2), st));
     k_bucket_count<<<G((int64_t)n * kRowLanes), kTB, 0, st>>>(h->csr_off, h->csr_col, n, keep, own, cnt);
     EGT_LAUNCH_CHECK();
     EGT_CUDA_TRY(cub::DeviceScan::ExclusiveSum(m + o_scan, t_scan, cnt, boff, n + 1, st));
-    k_bucket_fill<<<G((int64_t)n * kRowLanes), kTB, 0, st>>>(h->csr_off, h->csr_col, n, bits, keep, boff, own, key);
+    k_bucket_fill<<<G((int64_t)n * kRowLanes), kTB, 0, st>>>(h->csr_off, h->csr_col, n, bits, keep, boff, own, key, longs,
+                                                               n_long);
     EGT_LAUNCH_CHECK();
+    if (nnz > kLongBucket) {
+        const unsigned gl = (unsigned)std::min<int64_t>(nnz / kLongBucket, 148);
+        k_bucket_sort<<<gl, kRadixThreads, 0, st>>>(key, ukey, boff, longs, n_long, bits);
+        EGT_LAUNCH_CHECK();
+    }
     k_bucket_edges<<<G(nnz), kTB, 0, st>>>(key, boff, n, bits, h->nrm, ukey, act, sgn);
     EGT_LAUNCH_CHECK();
     // 2. Borůvka rounds (the unordered edges' buffer is free again)
