@@ -197,11 +197,14 @@ __global__ void k_head_flags64(const unsigned long long* __restrict__ key, int64
     flag[i] = (i == 0 || key[i] != key[i - 1]) ? 1 : 0;
 }
 
-// Per-cloud cell tables of one level (grid.cu k_cells per cloud slice).
+// Per-cloud cell tables of one level (grid.cu k_tables per cloud slice), and
+// whether a cell of the cloud is oversized: max_pts at kCtrMaxPop + L, else 0, which
+// is all that the searches compare a level's largest population with.  (A pass of
+// its own over the finished tables cost 3 to 6 % of a batch's creation.)
 __global__ void k_cells_batch(const unsigned long long* __restrict__ key, const int* __restrict__ flag,
                               const int* __restrict__ cid, const uint16_t* __restrict__ cloud,
                               const int64_t* __restrict__ off, int64_t N, int B, int L, int* __restrict__ cell_start,
-                              int* __restrict__ cell_x, int2* __restrict__ rows, int* __restrict__ cbase,
+                              int* __restrict__ cell_x, int2* __restrict__ rows, int* __restrict__ cbase, int max_pts,
                               unsigned long long* __restrict__ ctr) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= N) return;
@@ -221,6 +224,8 @@ __global__ void k_cells_batch(const unsigned long long* __restrict__ key, const 
         ctr[(size_t)c * kCtrWords + kCtrNcells + L] = (unsigned long long)nc;
     }
     if (!flag[i]) return;
+    if (i - o + max_pts <= nc_pts && key[i + max_pts - 1] == key[i])
+        ctr[(size_t)c * kCtrWords + kCtrMaxPop + L] = (unsigned long long)max_pts;
     const int lc = cid[i] - cb;
     const int slot = cid[i] + c;
     cell_start[slot] = (int)(i - o);
@@ -283,19 +288,6 @@ __global__ void k_make_desc(DescArgs d, KnnArgs* __restrict__ out) {
     a.maxpop = a.counters + kCtrMaxPop;
     a.gbase = o;
     out[c] = a;
-}
-
-// Largest cell population of each cloud and level (the searches' oversized-cell
-// check): blockIdx.x a slice of the cells, (y, z) the level and the cloud.
-constexpr int kPopSlices = 16;
-__global__ void __launch_bounds__(256) k_maxpop_batch(const KnnArgs* __restrict__ desc) {
-    const KnnArgs& a = desc[blockIdx.z];
-    const LevelDev& LV = a.lv[blockIdx.y];
-    int v = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < LV.ncells; i += kPopSlices * blockDim.x)
-        v = max(v, LV.cell_start[i + 1] - LV.cell_start[i]);
-    v = __reduce_max_sync(0xffffffffu, v);
-    if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(&a.counters[kCtrMaxPop + blockIdx.y], (unsigned long long)v);
 }
 
 __global__ void k_set_chunk(KnnArgs* __restrict__ desc, int count, int chunk) {
@@ -1000,7 +992,7 @@ egt_status egt_batch_create(const float* xyz_host, const int64_t* offsets, const
         BSTAT([&] { EGT_LAUNCH_CHECK(); return EGT_OK; }());
         BTRY(cub::DeviceScan::ExclusiveSum(tmp, t_scan, flag, cid, (int)N, st));
         k_cells_batch<<<blocks(N), kB, 0, st>>>(keys, flag, cid, b->d_cloud, b->d_off, N, B, L, b->cell_start[L],
-                                               b->cell_x[L], b->rows[L], b->cbase[L], b->d_ctr);
+                                               b->cell_x[L], b->rows[L], b->cbase[L], cfg.max_points_in_cell, b->d_ctr);
         BSTAT([&] { EGT_LAUNCH_CHECK(); return EGT_OK; }());
     }
     DescArgs da{};
@@ -1024,8 +1016,6 @@ egt_status egt_batch_create(const float* xyz_host, const int64_t* offsets, const
     da.qlevel = h->qlevel;
     da.ctr = b->d_ctr;
     k_make_desc<<<blocks(count), kB, 0, st>>>(da, b->d_desc);
-    BSTAT([&] { EGT_LAUNCH_CHECK(); return EGT_OK; }());
-    k_maxpop_batch<<<dim3(kPopSlices, kMaxLevels, (unsigned)count), 256, 0, st>>>(b->d_desc);
     BSTAT([&] { EGT_LAUNCH_CHECK(); return EGT_OK; }());
     BTRY(cudaEventRecord(h->ev[1], st));
     for (void* p : {(void*)dxyz, (void*)acc, (void*)tmp4, (void*)kA, (void*)kB2, (void*)iA, (void*)iB, (void*)flag,

@@ -20,7 +20,8 @@ struct KnnArgs {
     float* __restrict__ kth_out;
     uint8_t* __restrict__ qlevel;
     unsigned long long* __restrict__ counters;
-    const unsigned long long* __restrict__ maxpop = nullptr;  // [kMaxLevels] largest cell population of each level
+    // [kMaxLevels] largest cell population of each level (batches: max_pts where a cell holds as many, else 0)
+    const unsigned long long* __restrict__ maxpop = nullptr;
     const int* __restrict__ qmap = nullptr;  // query j of a launch is qmap[j] (nullptr: j)
     unsigned long long* __restrict__ work = nullptr;  // work counter (nullptr: counters[kCtrWork])
     const unsigned long long* __restrict__ n_dev = nullptr;  // launch size on the device (nullptr: n)
