@@ -33,6 +33,7 @@
 // memsets): 2,000 points 325 -> 76 us (host-bound before), 36K 603 -> 99 us, 1M
 // 836 -> 410 us, 4M 1.77 -> 1.40 ms, 20M 6.89 -> 6.77 ms.
 #include <algorithm>
+#include <cub/cub.cuh>
 #include "egt_internal.cuh"
 #include "grid_common.cuh"
 #include "radix.cuh"
@@ -45,6 +46,13 @@ constexpr int kL0Bits = 8;           // digits of the level-0 sort (30-bit keys)
 constexpr int kL0Passes = 4;
 constexpr int kLevelBits = kRadixBits;     // widest digit of the upper levels' sorts
 constexpr int kMaxPasses = 4;
+// Clouds of more points sort with the library after the first pass of each level,
+// as every cloud did before the shared passes: its passes move 2 TB/s of pairs there
+// against 1.6 (the votes of radix_peers bound a large pass), while the first
+// pass still forms the keys and the tables come from k_tables.  Build time, library
+// / this / own passes alone: sheets 20M 6.80 / 6.72 / 6.72 ms, 30M 9.95 / 9.70 / 10.19,
+// 40M 12.9 / 12.9 / 13.7, 80M 24.8 / 25.8 / 27.6.
+constexpr int64_t kLibrarySort = 24 << 20;
 constexpr int64_t kGroupBytes = 256 << 20;  // (key, value) pairs in and out of the levels sorted together
 
 // Digits of a level's sort: 3 (10 - L) key bits in passes of near-equal width.
@@ -434,7 +442,9 @@ egt_status build_grid(egt_handle* h, const float* xyz, int levels) {
     EGT_TRY(level_memory(h, levels));
     h->levels_built = levels;
     const int64_t tiles = radix_tiles(n), ttiles = (n + kTableTile - 1) / kTableTile;
-    const int group = (int)std::max<int64_t>(1, std::min<int64_t>(kMaxLevels - 1, kGroupBytes / (16 * n)));
+    const bool library = n > kLibrarySort;
+    const int group =
+        library ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(kMaxLevels - 1, kGroupBytes / (16 * n)));
     // scratch: what starts at zero (digit counts, look-back words, tickets), then the sorts' buffers
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t a = at; at += align256(bytes); return a; };
@@ -453,6 +463,11 @@ egt_status build_grid(egt_handle* h, const float* xyz, int levels) {
     const size_t o_key0 = take(sizeof(uint32_t) * n);
     const size_t o_buf = take(0), stride = align256(sizeof(uint32_t) * n);
     take(stride * 4 * group);
+    size_t t_sort = 0;
+    if (library)
+        EGT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, t_sort, (const uint32_t*)nullptr, (uint32_t*)nullptr,
+                                                     (const int*)nullptr, (int*)nullptr, (int)n, 0, 30, st));
+    const size_t o_sort = take(t_sort);
     void* mem = nullptr;
     EGT_TRY(scratch_reserve(h, at, &mem));
     char* m = static_cast<char*>(mem);
@@ -474,7 +489,14 @@ egt_status build_grid(egt_handle* h, const float* xyz, int levels) {
     RadixBatch rb{};
     rb.n = (int)n;
     rb.polls = kRadixPolls;
-    for (int p = 0; p < kL0Passes; p++) {
+    // the digits from bit `from` on of keys sorted by the digits below (a large cloud)
+    auto rest = [&](const uint32_t* key_in, uint32_t* key_out, const int* val_in, int* val_out, int from,
+                    int to) -> egt_status {
+        EGT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(m + o_sort, t_sort, key_in, key_out, val_in, val_out, (int)n, from,
+                                                     to, st));
+        return EGT_OK;
+    };
+    for (int p = 0; p < (library ? 1 : kL0Passes); p++) {
         RadixJob& j = rb.job[0];
         j.key_in = keys(0, p & 1);
         j.val_in = p ? vals(0, p & 1) : nullptr;
@@ -486,11 +508,12 @@ egt_status build_grid(egt_handle* h, const float* xyz, int levels) {
         j.shift = p * kL0Bits;
         j.bits = kL0Bits;
         j.xf = kKeyRaw;
-        j.next_hist = p + 1 < kL0Passes ? U(o_hist0) + ((p + 1) << kL0Bits) : nullptr;
+        j.next_hist = p + 1 < kL0Passes && !library ? U(o_hist0) + ((p + 1) << kL0Bits) : nullptr;
         j.next_shift = j.shift + kL0Bits;
         j.next_bits = kL0Bits;
         EGT_TRY(radix_pass(rb, 1, st));
     }
+    if (library) EGT_TRY(rest(keys(0, 1), U(o_key0), vals(0, 1), h->perm, kL0Bits, 30));
     EGT_TRY(launch_dependent(k_gather_sorted, dim3(gk), dim3(kT), 0, st, xyz, h->perm, U(o_key0), n, h->p4, h->x, h->y,
                              h->z, h->cell0, h->d_norm, levels > 1 ? U(o_hist) : nullptr));
     TableBatch tb{};
@@ -506,10 +529,10 @@ egt_status build_grid(egt_handle* h, const float* xyz, int levels) {
     tb.job[tjobs++] = table(0, U(o_key0));
     for (int L0 = 1; L0 < levels || tjobs; L0 += group) {
         const int L1 = std::min(levels, L0 + group);  // levels [L0, L1) are sorted together
-        for (int p = 0; p < kMaxPasses; p++) {
+        for (int p = 0; p < (library ? 1 : kMaxPasses); p++) {
             int jobs = 0;
             for (int L = L0; L < L1 && level_passes(L) > p; L++) {
-                const int g = L - L0, last = level_passes(L) - 1;
+                const int g = L - L0, last = library ? kMaxPasses : level_passes(L) - 1;  // the pass that ends in the tables
                 RadixJob& j = rb.job[jobs++];
                 // A, B, A...: a pass never writes what it reads
                 j.key_in = p ? keys(g, (p - 1) & 1) : h->cell0;
@@ -522,12 +545,16 @@ egt_status build_grid(egt_handle* h, const float* xyz, int levels) {
                 j.shift = pass_shift(L, p);
                 j.bits = pass_bits(L, p);
                 j.xf = p ? kKeyRaw : L;
-                j.next_hist = p < last ? U(o_hist) + ((size_t)hist_slot(L, p + 1) << kLevelBits) : nullptr;
-                j.next_shift = p < last ? pass_shift(L, p + 1) : 0;
-                j.next_bits = p < last ? pass_bits(L, p + 1) : 0;
+                j.next_hist = p < last && !library ? U(o_hist) + ((size_t)hist_slot(L, p + 1) << kLevelBits) : nullptr;
+                j.next_shift = j.next_hist ? pass_shift(L, p + 1) : 0;
+                j.next_bits = j.next_hist ? pass_bits(L, p + 1) : 0;
                 if (p == last) tb.job[tjobs++] = table(L, keys(g, p & 1));
             }
             if (jobs) EGT_TRY(radix_pass(rb, jobs, st));
+        }
+        if (library && L0 < levels) {  // one level at a time
+            EGT_TRY(rest(keys(0, 0), keys(0, 1), vals(0, 0), h->lv[L0].order, pass_bits(L0, 0), level_bits(L0)));
+            tb.job[tjobs++] = table(L0, keys(0, 1));
         }
         EGT_TRY(launch_dependent(k_tables, dim3((unsigned)ttiles, (unsigned)tjobs), dim3(kT), 0, st, tb));
         tjobs = 0;
