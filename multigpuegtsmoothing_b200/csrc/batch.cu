@@ -743,11 +743,14 @@ egt_status taubin_batch(egt_batch* b, int iters, float lambda, float mu) {
 }
 
 // Autotuner: times each kNN work chunk and each Taubin half-step kernel on the
-// batch itself; results are cached per (log2 points, max k) bucket.
+// batch itself; results are cached per (log2 points, max k) bucket, and on which
+// side of the resident loop's size it lies: there the staged tiles are another
+// kernel.
 struct TuneKey {
     int device, logn, kmax;
+    bool one_launch;
     bool operator<(const TuneKey& o) const {
-        return std::tie(device, logn, kmax) < std::tie(o.device, o.logn, o.kmax);
+        return std::tie(device, logn, kmax, one_launch) < std::tie(o.device, o.logn, o.kmax, o.one_launch);
     }
 };
 std::mutex g_tune_mu;
@@ -758,7 +761,9 @@ std::map<TuneKey, TuneVal> g_tune;
 
 egt_status autotune(egt_batch* b, float lambda, float mu, float alpha) {
     if (b->tuning_fixed || b->chunk > 0) return EGT_OK;
-    const TuneKey key{b->cfg.device, (int)std::lround(std::log2((double)b->N)), b->kmax};
+    bool one_launch = false;
+    EGT_TRY(taubin_one_launch(b->N, &one_launch));
+    const TuneKey key{b->cfg.device, (int)std::lround(std::log2((double)b->N)), b->kmax, one_launch};
     {
         std::lock_guard<std::mutex> lock(g_tune_mu);
         auto it = g_tune.find(key);

@@ -889,6 +889,48 @@ static egt_status scatter_launch(egt_handle* h, cudaStream_t st) {
                             n, h->p4, h->x, h->y, h->z, h->cell0);
 }
 
+// Blocks of one resident wave of the staged half-step and of the whole loop on the
+// current device.
+static egt_status loop_waves(unsigned* staged, unsigned* whole) {
+    // function attributes are per device: set them once on each, and size the
+    // persistent grid from the occupancy they allow
+    static std::atomic<uint64_t> attr_set{0};
+    static std::atomic<unsigned> wave[64], resident[64];
+    int dev = 0;
+    EGT_CUDA_TRY(cudaGetDevice(&dev));
+    if (!(attr_set.load() >> (dev & 63) & 1)) {
+        EGT_CUDA_TRY(cudaFuncSetAttribute(k_taubin_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPipeSmem));
+        // the whole unified L1/shared array as shared memory, so that four
+        // 50-KB blocks fit on an SM
+        EGT_CUDA_TRY(cudaFuncSetAttribute(k_taubin_tiles, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                          (int)cudaSharedmemCarveoutMaxShared));
+        int sms = 0, per = 0;
+        EGT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        EGT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_taubin_tiles, kTile, kPipeSmem));
+        wave[dev & 63].store((unsigned)std::max(1, sms * std::max(per, 1)));
+        EGT_CUDA_TRY(cudaFuncSetAttribute(k_taubin_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)kResidentSmem));
+        EGT_CUDA_TRY(cudaFuncSetAttribute(k_taubin_resident, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                          (int)cudaSharedmemCarveoutMaxShared));
+        EGT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_taubin_resident, kTile, kResidentSmem));
+        resident[dev & 63].store((unsigned)(sms * per));
+        attr_set.fetch_or(uint64_t(1) << (dev & 63));
+    }
+    *staged = wave[dev & 63].load();
+    *whole = resident[dev & 63].load();
+    return EGT_OK;
+}
+
+// Whether a cloud of n points is small enough for the resident loop (its tiles
+// have to be staged, too).
+egt_status taubin_one_launch(int64_t n, bool* out) {
+    unsigned staged = 0, whole = 0;
+    EGT_TRY(loop_waves(&staged, &whole));
+    const int64_t tiles = (n + kTile - 1) / kTile;
+    *out = tiles <= kResidentMaxTiles && tiles <= (int64_t)whole;
+    return EGT_OK;
+}
+
 egt_status run_taubin(egt_handle* h, int iters, float lambda, float mu) {
     if (iters < 0) { set_error("egt_taubin: iters must be >= 0"); return EGT_ERR_ARG; }
     if (!h->lists) { set_error("egt_taubin: no neighbour lists"); return EGT_ERR_STATE; }
@@ -898,36 +940,11 @@ egt_status run_taubin(egt_handle* h, int iters, float lambda, float mu) {
     EGT_CUDA_TRY(cudaEventRecord(h->ev[6], st));
     if (iters > 0) {
         EGT_TRY(morton_prepare(h));
-        // function attributes are per device: set them once on each, and size
-        // the persistent grid from the occupancy they allow
-        static std::atomic<uint64_t> attr_set{0};
-        static std::atomic<unsigned> wave[64], resident[64];  // blocks of one resident wave
-        int dev = 0;
-        EGT_CUDA_TRY(cudaGetDevice(&dev));
-        if (!(attr_set.load() >> (dev & 63) & 1)) {
-            EGT_CUDA_TRY(cudaFuncSetAttribute(k_taubin_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)kPipeSmem));
-            // the whole unified L1/shared array as shared memory, so that four
-            // 50-KB blocks fit on an SM
-            EGT_CUDA_TRY(cudaFuncSetAttribute(k_taubin_tiles, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                              (int)cudaSharedmemCarveoutMaxShared));
-            int sms = 0, per = 0;
-            EGT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-            EGT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_taubin_tiles, kTile, kPipeSmem));
-            wave[dev & 63].store((unsigned)std::max(1, sms * std::max(per, 1)));
-            EGT_CUDA_TRY(cudaFuncSetAttribute(k_taubin_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)kResidentSmem));
-            EGT_CUDA_TRY(cudaFuncSetAttribute(k_taubin_resident, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                              (int)cudaSharedmemCarveoutMaxShared));
-            EGT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_taubin_resident, kTile, kResidentSmem));
-            resident[dev & 63].store((unsigned)(sms * per));
-            attr_set.fetch_or(uint64_t(1) << (dev & 63));
-        }
-        const unsigned blocks = wave[dev & 63].load();
+        unsigned blocks = 0, whole = 0;
+        EGT_TRY(loop_waves(&blocks, &whole));
         const int tiles = (n + kTile - 1) / kTile;
         int64_t spilled = 1;
-        if (h->taubin_mode == 0 && h->t_adj && tiles <= (int)resident[dev & 63].load())
-            EGT_TRY(spilled_tiles(h, &spilled));
+        if (h->taubin_mode == 0 && h->t_adj && tiles <= (int)whole) EGT_TRY(spilled_tiles(h, &spilled));
         if (spilled == 0) {
             int left = 0;
             EGT_TRY(resident_loop(h, iters, lambda, mu, st, &left));
