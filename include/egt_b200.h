@@ -100,9 +100,12 @@ typedef struct egt_timings {
     int64_t taubin_tiles;    /* 256-row tiles of the staged Taubin half-step (last CSR smoothed) */
     int64_t taubin_spill_tiles; /* of those, tiles too large to stage in shared memory, whose rows
                                    gather their neighbours from global memory */
-    int64_t knn_fallback;    /* EGT_KNN_SELECT / EGT_KNN_TILE: queries the block selection or the cell
-                                tiles did not certify (equal distances, oversized cells, a k-th ball
-                                beyond the block, ...) or did not take, which the ring search ran */
+    int64_t knn_fallback;    /* EGT_KNN_SELECT / EGT_KNN_TILE: queries the ring search ran because the block
+                                selection or the cell tiles did not certify them (equal distances,
+                                oversized cells, a k-th ball beyond the block, ...) or did not take them;
+                                the same after egt_knn and egt_knn_host.  EGT_KNN_TILE: all of a cloud
+                                too small for the tiles where 16 <= k <= 64; 0 where k is outside that
+                                range and the tiles were not taken */
 } egt_timings;
 
 void egt_default_config(egt_config* cfg);

@@ -877,6 +877,12 @@ static egt_status tile_search(egt_handle* h, const KnnArgs& a, cudaStream_t st) 
 // Whether EGT_KNN_TILE takes the cell-tile search.
 bool knn_tiles(int64_t n, int k) { return tile_takes(n, k); }
 
+// Notes for egt_timings::knn_fallback whether the ring search runs every row of a
+// search whose k is the tiles' (the cloud is too small for them).
+static void note_untiled(egt_handle* h, int k) {
+    h->knn_untiled = h->cfg.knn_mode == EGT_KNN_TILE && k >= kTileLowK && k <= kTileMaxK && !tile_takes(h->n, k);
+}
+
 egt_status run_knn(egt_handle* h, int k) {
     cudaStream_t st = h->stream;
     KnnArgs a;
@@ -884,7 +890,7 @@ egt_status run_knn(egt_handle* h, int k) {
     EGT_TRY(reset_knn_counters(h));
     EGT_CUDA_TRY(cudaEventRecord(h->ev[2], st));
     const bool tile = h->cfg.knn_mode == EGT_KNN_TILE;
-    h->knn_untiled = tile && k >= kTileLowK && k <= kTileMaxK && !tile_takes(h->n, k);
+    note_untiled(h, k);
     if (tile && tile_takes(h->n, k)) EGT_TRY(tile_search(h, a, st));
     else EGT_TRY(knn_search(a, h->cfg.knn_mode == EGT_KNN_SELECT, jump_queries(h), st));
     EGT_CUDA_TRY(cudaEventRecord(h->ev[3], st));
@@ -946,9 +952,9 @@ __global__ void k_rows_original(const int* __restrict__ lists, const int* __rest
 // them.
 egt_status run_knn_host(egt_handle* h, int k, int* host) {
     cudaStream_t st = h->stream;
-    h->knn_untiled = false;
     KnnArgs a;
     EGT_TRY(knn_prepare(h, k, &a));
+    note_untiled(h, k);
     const int n = (int)h->n;
     ChunkBounds cb{};
     {
