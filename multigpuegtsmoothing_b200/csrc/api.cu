@@ -572,10 +572,12 @@ egt_status egt_copy_to_host(egt_handle* h, void* dst, const void* src, int64_t b
 }
 
 // For the tests (not in the header): the polls after which a wait of the
-// resident Taubin loop gives up (0: the default), and one of the handle's counters.
-egt_status egt_internal_set_polls(egt_handle* h, int resident) {
+// resident Taubin loop (0: the default) and of a look-back of the grid build (-1:
+// the default) gives up, and one of the handle's counters.
+egt_status egt_internal_set_polls(egt_handle* h, int resident, int lookback) {
     EGT_TRY(check_handle(h));
     h->resident_polls = resident;
+    h->lookback_polls = lookback;
     return EGT_OK;
 }
 int64_t egt_internal_counter(egt_handle* h, int word) {

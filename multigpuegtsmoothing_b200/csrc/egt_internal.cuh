@@ -132,7 +132,7 @@ constexpr int kMaxLevels = 8;  // levels 0..7 (B = 1024 .. 8) are searched
 // Layout of egt_handle::d_counters (unsigned long long words).
 constexpr int kCtrWords = 64;
 constexpr int kCtrNcells = 0;     // [0..7]  occupied cells per level (int in a u64 slot)
-constexpr int kCtrExtents = 16;   // [16..18] six packed u32 min/max words
+constexpr int kCtrRecounts = 16;  // grid build: tiles whose look-back expired and that counted for themselves
 constexpr int kCtrEgtTests = 24;    // EGT filter: ellipsoid tests of the last filter run
 constexpr int kCtrSpillTiles = 25;  // Taubin tiles that gather from global memory (too large to stage)
 constexpr int kCtrTaubinFail = 26;  // a wait of the resident Taubin loop expired (until it is redone)
@@ -197,6 +197,7 @@ struct egt_handle {
     void* grid_mem = nullptr;    // row ranges of all levels, then their cells and orders
     size_t row_bytes = 0;        // bytes of the row ranges
     int levels_built = 0;
+    int lookback_polls = -1;     // polls of one look-back word of the grid build (-1: kRadixPolls)
     // neighbourhoods
     int* lists = nullptr;        // [n*k] sorted-space lists
     float* kth = nullptr;        // [n] k-th distance per query (diagnostics / learned labels)

@@ -325,6 +325,7 @@ __global__ void __launch_bounds__(kT) k_tables(const __grid_constant__ TableBatc
         if (lane == 0) { s_prev = prev; s_plast = plast; }
     }
     if (__syncthreads_or(lost)) {  // a predecessor did not answer: count its heads here
+        if (threadIdx.x == 0) atomicAdd(&b.counters[kCtrRecounts], 1ull);
         uint32_t c = 0, l = 0;
         for (int64_t i = threadIdx.x; i < first; i += kT)
             if (is_head(i)) { c++; l = (uint32_t)i + 1u; }
@@ -488,7 +489,8 @@ egt_status build_grid(egt_handle* h, const float* xyz, int levels) {
     EGT_TRY(launch_dependent(k_keys, dim3(gk), dim3(kT), 0, st, xyz, n, h->d_norm, keys(0, 0), U(o_hist0)));
     RadixBatch rb{};
     rb.n = (int)n;
-    rb.polls = kRadixPolls;
+    rb.polls = h->lookback_polls >= 0 ? h->lookback_polls : kRadixPolls;
+    rb.recounts = h->d_counters + kCtrRecounts;
     // the digits from bit `from` on of keys sorted by the digits below (a large cloud)
     auto rest = [&](const uint32_t* key_in, uint32_t* key_out, const int* val_in, int* val_out, int from,
                     int to) -> egt_status {
@@ -518,7 +520,7 @@ egt_status build_grid(egt_handle* h, const float* xyz, int levels) {
                              h->z, h->cell0, h->d_norm, levels > 1 ? U(o_hist) : nullptr));
     TableBatch tb{};
     tb.n = (int)n;
-    tb.polls = kRadixPolls;
+    tb.polls = rb.polls;
     tb.counters = h->d_counters;
     auto table = [&](int L, const uint32_t* key) {
         const LevelDev& lv = h->lv[L];

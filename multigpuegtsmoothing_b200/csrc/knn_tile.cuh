@@ -92,6 +92,8 @@ constexpr int kTileSparse = 2;       // a finer block below (k+1)/kTileSparse po
                                       // on 4M superquadrics at k = 40: (k+1)/2 and 0.6(k+1) best, 0.75(k+1)
                                       // 8 % slower, 0.45(k+1) and below 15 % slower: its long searches return)
 constexpr int kTileMaxBlock = 6144;   // larger blocks: the ring search (one warp would hold the search's end)
+static_assert(kTileMaxBlock <= 1 << kTilePosBits, "block positions fit their bits");
+static_assert(kTileMaxBlock <= 128 * 4 * 16, "the step groups of a block fit the half's 128 bytes");
 constexpr int kTileStartLevel = 3;   // the assignment's first level (the usual one on dense clouds)
 constexpr int kTileClasses = 6;       // batch classes by block size (>= 4096, 2048, 1024, 512, 256, less)
 
@@ -107,9 +109,8 @@ struct TileArgs {
     int maxblock;                     // kTileMaxBlock
     uint32_t* qarr;                   // [n] the units' queries, grouped by unit (k_tile_gather)
     unsigned long long* n_q;          // queries written to qarr
-    uint2* batch;                     // [bcap] (unit index, first query in qarr), largest blocks first
-    uint8_t* bcnt;                    // [bcap] queries in each batch (1..16)
-    int bcap;                         // n + n/16 + 1 >= units + queries/16
+    uint2* batch;                     // [n + n/16 + 1 >= units + queries/16] (unit index, first query in qarr), largest blocks first
+    uint8_t* bcnt;                    // [the same] queries in each batch (1..16)
     uint32_t* ucnt;                   // [n] queries of each unit
     uint8_t* ucls;                    // [n] class of each unit's block
     unsigned long long* cls_n;        // [kTileClasses] batches per class
@@ -981,7 +982,6 @@ inline egt_status tile_prepare(egt_handle* h, TileArgs* t) {
     t->bcnt = m;
     m += b_bcnt;
     t->ucls = m;
-    t->bcap = (int)bcap;
     t->n_units = h->d_counters + kCtrTileUnits;
     t->unit_work = h->d_counters + kCtrTileWork;
     t->n_ring = h->d_counters + kCtrSelFallback;

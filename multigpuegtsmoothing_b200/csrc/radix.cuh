@@ -37,31 +37,15 @@ constexpr uint32_t kStateSum = 1u << 30;   // the word holds the tile's own coun
 constexpr uint32_t kStateFull = 2u << 30;  // the word holds the count up to and including the tile
 constexpr uint32_t kStateValue = kStateSum - 1;
 
-// 30-bit Morton code of a packed level-0 cell (x | y<<10 | z<<20).
-__device__ __forceinline__ uint32_t spread3(uint32_t v) {
-    v &= 0x3ffu;
-    v = (v | (v << 16)) & 0x030000ffu;
-    v = (v | (v << 8)) & 0x0300f00fu;
-    v = (v | (v << 4)) & 0x030c30c3u;
-    v = (v | (v << 2)) & 0x09249249u;
-    return v;
-}
-__device__ __forceinline__ uint32_t morton_key(uint32_t c) {
-    return spread3(c) | (spread3(c >> 10) << 1) | (spread3(c >> 20) << 2);
-}
 // Key x + y*B + z*B^2 of the level-L cell of a packed level-0 cell.
 __device__ __forceinline__ uint32_t level_key(uint32_t c, int L) {
     const int b = 10 - L;
     return ((c & 1023u) >> L) | ((((c >> 10) & 1023u) >> L) << b) | (((c >> 20) & 1023u) >> L) << (2 * b);
 }
 
-constexpr int kKeyRaw = -1;     // the keys themselves
-constexpr int kKeyMorton = 16;  // packed level-0 cells, sorted by Morton code
-                                // 1..7: packed level-0 cells, sorted by their level-L cell
+constexpr int kKeyRaw = -1;  // the keys themselves (1..7: packed level-0 cells, sorted by their level-L cell)
 
-__device__ __forceinline__ uint32_t radix_key(uint32_t v, int xf) {
-    return xf == kKeyRaw ? v : xf == kKeyMorton ? morton_key(v) : level_key(v, xf);
-}
+__device__ __forceinline__ uint32_t radix_key(uint32_t v, int xf) { return xf == kKeyRaw ? v : level_key(v, xf); }
 
 struct RadixJob {
     const uint32_t* key_in;  // keys, or what they are formed from (xf)
@@ -78,7 +62,8 @@ struct RadixJob {
 struct RadixBatch {
     RadixJob job[kRadixJobs];
     int n;
-    int polls;  // kRadixPolls
+    int polls;                    // kRadixPolls
+    unsigned long long* recounts;  // tiles that counted for themselves
 };
 
 // Exclusive prefix of one value per thread over the block.  s: kRadixWarps
@@ -227,6 +212,7 @@ __global__ void __launch_bounds__(kRadixThreads, 4) k_radix_pass(const __grid_co
         }
     }
     if (__syncthreads_or(lost)) {  // a predecessor did not answer: count its elements here
+        if (d == 0) atomicAdd(b.recounts, 1ull);
         uint32_t* all = reinterpret_cast<uint32_t*>(&s_cnt[0][0]);
         all[d] = 0u;
         __syncthreads();

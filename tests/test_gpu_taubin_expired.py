@@ -21,7 +21,7 @@ def _counter(lib, handle, word):
 @pytest.mark.parametrize("n,iters", [(2500, 7), (36001, 5)])
 def test_expired_wait_is_computed_again(capi, n, iters):
     lib = capi.lib()
-    lib.egt_internal_set_polls.argtypes = [C.c_void_p, C.c_int]
+    lib.egt_internal_set_polls.argtypes = [C.c_void_p, C.c_int, C.c_int]
     xyz = datagen.sphere_cloud(n, 0.005, n)
     out = []
     for polls in (0, 1):
@@ -29,12 +29,12 @@ def test_expired_wait_is_computed_again(capi, n, iters):
         g.GRIDCUDAKNNSELF_COMPACT(24)
         egt = capi.EGT_CUDA(g)
         egt.Filter(0.65)
-        lib.egt_internal_set_polls(g.handle, polls)
+        lib.egt_internal_set_polls(g.handle, polls, -1)
         egt.Taubin(iters, 0.63, -0.64)
         first = g.sorted_positions()
         redone = _counter(lib, g.handle, REDONE)
         assert redone == 0 if polls == 0 else redone == 1
-        lib.egt_internal_set_polls(g.handle, 0)
+        lib.egt_internal_set_polls(g.handle, 0, -1)
         egt.Taubin(iters, 0.63, -0.64)  # the next loop is not touched by the expired one
         g.timings()
         assert _counter(lib, g.handle, REDONE) == redone
