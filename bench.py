@@ -372,8 +372,7 @@ def learned_compare(capi, xyz, k, train, workload):
            "block_selection_ms": min(select_ms), "block_selection_mqueries_s": n / min(select_ms) / 1e3,
            "block_selection_note": "the block-selection search (EGT_KNN_SELECT) on the same cloud, same lists",
            "tile_ms": min(tile_ms), "tile_mqueries_s": n / min(tile_ms) / 1e3,
-           "tile_note": "the cell-tile search (EGT_KNN_TILE, egt_knn's default; the ring search for k outside "
-                        "16..64) on the same cloud, same lists"}
+           "tile_note": "the cell-tile search (EGT_KNN_TILE, egt_knn's default) on the same cloud, same lists"}
     g.close()
     p.close()
     return out
@@ -605,7 +604,7 @@ def run_b200(args, world, rank, local):
         barrier(world)
         s = time.perf_counter()
         h2 = capi.GridStructure(host_xyz.numpy())
-        h2.knn_host(K, out=host_knn.numpy())  # search + original-order lists to host, copies overlapped
+        h2.knn_host(K, out=host_knn.numpy())  # search, then original-order lists to host
         h2.close()
         e = time.perf_counter() - s
         if i >= args.warmup:

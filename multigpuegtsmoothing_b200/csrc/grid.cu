@@ -20,8 +20,9 @@
 // rounding; the hierarchy therefore never re-reads positions.
 //
 // The build is a chain of 12 launches for a small cloud: extents, keys, four
-// radix passes (radix.cuh), gather, four passes that sort every level, and one that writes every level's tables (head
-// flags, cell numbering by look-back, row ranges and largest population).
+// radix passes (radix.cuh), gather, four passes that sort every level, and one
+// that writes every level's tables (head flags, cell numbering by look-back, row
+// ranges and largest population).
 // The levels of clouds of up to 2.4M points share their launches (kGroupBytes
 // of buffers), so that one level's waits are filled by the others' work; larger
 // clouds sort fewer at a time (4M points 1.40 ms so, 1.36 ms with all levels

@@ -51,7 +51,7 @@ namespace egt {
 namespace {
 
 constexpr int kTileWarps = 1;    // warps per block (one: blocks pack the SM's shared memory tightly)
-constexpr int kTileBins = 64;    // distance buckets per query: 8 per octave of d^2, (h/4)^2 to (4h)^2
+constexpr int kTileBins = 64;    // distance buckets per query: 8 per octave of d^2, placed by tile_unit_setup
 // Forms of the search by k: list registers S of the in-kernel ring search
 // (k+1 <= 32 S) and words kept per query, the query included (kKeep): k+2 and
 // the rest of the last bucket, which is 9 % of the count below it on a surface.
@@ -478,7 +478,7 @@ __device__ __forceinline__ void tile_distances(const float* stage, float4 pq, fl
 }
 
 // Batcher's merge exchange (Knuth, The Art of Computer Programming, vol. 3,
-// algorithm 5.2.2M) for N elements: 32: 191 comparators, 56: 462, 80: 842.
+// algorithm 5.2.2M) for N elements: 32: 191 comparators, 56: 464, 80: 849.
 template <int N>
 struct SortNet {
     static constexpr int count() {
@@ -648,8 +648,9 @@ __device__ __forceinline__ void tile_unit_setup(const KnnArgs& a, const NormPara
 // Persistent: each half-warp claims batches (up to 16 queries of one unit)
 // one at a time; both halves run their batches together.
 //
-// Bound: latency with few warps (a block of ~600 candidates is streamed twice
-// from shared memory, 16 at a time), then instruction issue.  Before the kept
+// Bound: instruction issue (64 % busy at 20 warps per SM, 1,104 instructions a
+// query of 1M superquadrics) and the latency of a block's stream (~600 candidates
+// twice from shared memory, 16 at a time).  Before the kept
 // candidates became one word each and were sorted by a network, 35 % of the
 // time went to fetching their distances again and to insertion sorts whose
 // steps differ from lane to lane, 29 % to the bucket places of pass 2.  One

@@ -16,7 +16,8 @@
 //
 // Bound: the latency of a pass (load, rank, look-back, scatter): 7 us for 36K
 // pairs, 45 us for 4M (1.4 TB/s) on their own, 42 us each when several sorts
-// share a launch and fill one another's waits.
+// share a launch and fill one another's waits; from tens of millions of pairs on
+// issue (55 to 65 % busy, DRAM a quarter of its peak; 1.6 TB/s).
 //
 // A look-back that waits too long (kRadixPolls) stops waiting: the block then
 // counts the elements before its tile from the pass's input, which no block
