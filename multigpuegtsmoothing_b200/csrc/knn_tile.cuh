@@ -681,7 +681,10 @@ __global__ void __launch_bounds__(kTileWarps * 32, Form::kWarps) k_knn_tile(KnnA
     // batches, so that the long ones do not end the search.  Its scratch lies
     // in the bucket space.  (Queries that fail the checks run it in a
     // separate launch at the ring kernel's own occupancy: measured faster than
-    // running them here, between batches.)
+    // running them here, between batches.)  It walks level by level: these queries
+    // lie alone beside dense cells, whose points the finer levels' neighbours keep
+    // out of the list; a jump meets them with an empty one (half of 200,000 points in
+    // a dense ball, k = 40: 1.28 ms against 1.50 with the jump; 4M superquadrics 8.4 both).
     int* r_pref = reinterpret_cast<int*>(hist);
     int* r_start = r_pref + 32;
     float* r_md = reinterpret_cast<float*>(r_start + 32);
@@ -694,8 +697,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, Form::kWarps) k_knn_tile(KnnA
         const NormParams np = *A.np;
         WarpList<S> L;
         bool invalid, rerun;
-        const int reached = plain_query<true, true, S>(A, np, q, A.p4[q], L, invalid, lane, r_pref, r_start, r_md,
-                                                       r_mp, rerun);
+        const int reached = plain_query<true, false, S>(A, np, q, A.p4[q], L, invalid, lane, r_pref, r_start, r_md,
+                                                        r_mp, rerun);
         write_query<S>(A, q, L, invalid, reached, lane);
         if constexpr (kBatch) {
             if (rerun && lane == 0) atomicAdd(&A.counters[kCtrExactRerun], 1ull);
