@@ -648,7 +648,7 @@ __device__ __forceinline__ void tile_unit_setup(const KnnArgs& a, const NormPara
 // Persistent: each half-warp claims batches (up to 16 queries of one unit)
 // one at a time; both halves run their batches together.
 //
-// Bound: instruction issue (64 % busy at 20 warps per SM, 1,104 instructions a
+// Bound: instruction issue (64 % busy at 20 warps per SM, 1,113 instructions a
 // query of 1M superquadrics) and the latency of a block's stream (~600 candidates
 // twice from shared memory, 16 at a time).  Before the kept
 // candidates became one word each and were sorted by a network, 35 % of the
